@@ -151,48 +151,6 @@ void LaunchLdlTrsm(const FactorFront<R>* fronts, const int2* tasks, int n, int J
 
 // ------------------------------------------------------------------ panel solves
 
-// One front of the panel being solved (cliq::Solve replacement, sweep.cu).
-template <typename R>
-struct SweepFront {
-    const cpx<R>* G;      // (s+u) x s selectively inverted factor, ld = ldg
-    const cpx<R>* D;      // pivots
-    cpx<R>* Rb;           // [s+u][3][k]: natural rhs, child 0 update, child 1 update
-    cpx<R>* parentRb;     // the parent's Rb (null for a root)
-    cpx<R>* Y;            // [s][k] forward result
-    cpx<R>* Z;            // [s+u][k] backward input
-    const int* lower;     // u ND indices of the front's structure
-    const int* rel;       // u rows of the structure in the parent front
-    int s, u, ndOff, childSlot;
-    int ldg;              // leading dimension of G (even)
-    const void* tmap;     // complex single: TMA maps of G (forward, backward; 128 bytes each)
-};
-
-// One CTA of a sweep launch: kSweepRows output rows from row0, kSweepCols
-// right-hand sides from col0, the K-chunk [k0, k1); split `split` of `nsplit`
-// whose partials live at slot+split and whose arrival counter is `counter`.
-struct SweepTile {
-    int front, row0, col0, k0, k1, split, nsplit, slot, counter;
-};
-
-constexpr int kSweepRows = 64;     // output rows per CTA (one per thread of a slice)
-constexpr int kSweepSlices = 4;    // K-slices per CTA, one warp pair each
-constexpr int kSweepThreads = kSweepRows * kSweepSlices;
-constexpr int kSweepCols = 16;
-constexpr size_t kSweepSmemBytes = 32 * 1024;  // staged right-hand-side chunk
-
-constexpr int kTcRows = 128;       // rows per CTA of the tensor-core sweep kernels (UMMA M)
-
-// Device scratch of the sweep: split-K partials (rows-per-tile * kSweepCols
-// complex entries per slot), arrival counters (zero between launches), the
-// panel's ND-ordered solution vector [ND index][k] and a status word (bit 2:
-// a tensor-core pipeline wait timed out).
-struct SweepWork {
-    void* partials;
-    int* counters;
-    void* xnd;
-    int* status;
-};
-
 struct PanelIO {
     const int* ndToNat;
     int nxy, nx, nz;
@@ -205,41 +163,83 @@ struct PanelIO {
     StencilParams sp;
 };
 
-// Largest K-chunk a sweep CTA can stage.
-template <typename R>
-int SweepMaxChunk();
-// Sets kernel attributes the sweep kernels need (call before any graph capture).
-template <typename R>
-void PrepareSweepKernels();
-// tasks: (front, first row), kSweepRows rows each.  `pdl`: launch as a
-// programmatic dependent of the preceding kernel (the tensor-core sweep).
-template <typename R>
-void LaunchSweepPregather(const SweepFront<R>* fr, const int2* tasks, int n, const z64* B, int k, const PanelIO& io,
-                          cudaStream_t st, bool pdl = false);
-template <typename R>
-void LaunchSweepForward(const SweepFront<R>* fr, const SweepTile* tiles, int n, int maxChunk, int k,
-                        const SweepWork& w, cudaStream_t st);
-template <typename R>
-void LaunchSweepBackwardGather(const SweepFront<R>* fr, const int2* tasks, int n, int k, const SweepWork& w,
-                               cudaStream_t st, bool pdl = false);
-template <typename R>
-void LaunchSweepBackward(const SweepFront<R>* fr, const SweepTile* tiles, int n, int maxChunk, z64* B, int k,
-                         const PanelIO& io, const SweepWork& w, cudaStream_t st);
+// One panel solve as two launches (sweep_flow.cu): the panel's right-hand
+// sides in the subproblem's ordering, then the whole elimination tree, forward
+// and backward, as one ordered tile list (cliq::Solve replacement).
 
-// Tensor-core (tcgen05, split TF32) forms for complex-single factors
-// (sweep_tc.cu); tiles of kTcRows rows, any K-chunk length, and `cols` (16
-// or 32) right-hand sides per tile: the tile list's col0 steps by `cols`,
-// and a split tile's partial slots and counters are per 16-column sub-tile
-// (slot (t.slot + split) * cols / 16 + h, counter t.counter * cols / 16 + h).
-void PrepareSweepTcKernels();
-// Bytes of the two TMA maps of one front, and their encoding (host) into
-// out (64-byte aligned host memory) for the front's G, s, u and ldg.
-constexpr size_t kSweepTcMapBytes = 256;
-void EncodeSweepTcMaps(const SweepFront<float>& f, void* out);
-void LaunchSweepForwardTc(const SweepFront<float>* fr, const SweepTile* tiles, int n, int k, int cols,
-                          const SweepWork& w, cudaStream_t st);
-void LaunchSweepBackwardTc(const SweepFront<float>* fr, const SweepTile* tiles, int n, z64* B, int k, int cols,
-                           const PanelIO& io, const SweepWork& w, cudaStream_t st);
+constexpr int kFlowStageK = 16;    // K columns per stage of a tile
+constexpr int kFlowMaxCols = 32;   // right-hand sides per tile
+constexpr size_t kFlowMapBytes = 256;  // the two TMA maps of one front
+constexpr int kTcRows = 128;       // rows of a tensor-core tile (UMMA M)
+// Right-hand sides from which the tensor-core kernel is the faster one: its
+// time hardly depends on their number (96 x 96 x 76: 11.3 ms per sweep at 1 to 4,
+// 11.8 at 8), the CUDA-core kernel takes 7.5, 8.7 and 12.1 ms at 1, 2 and 4.
+constexpr int kFlowTcMinCols = 3;
+// Rows of a tile: a stage of G is 16 KB.
+template <typename R>
+constexpr int FlowRows() { return 1024 / (int)sizeof(cpx<R>); }
+
+// One front of the panel being solved (copied in 16-byte words).
+template <typename R>
+struct alignas(16) FlowFront {
+    const cpx<R>* D;      // pivots
+    cpx<R>* Pp;           // the parent's plane [s+u][k] that this front's update rows go to
+    const cpx<R>* P0;     // the planes its own children write (null: no child, or one without pivots);
+    const cpx<R>* P1;     // rows a child does not write are zero
+    const int* rel;       // u entries: row of each update row in the parent
+    const int* lower;     // u indices of the front's structure in the subproblem's ordering
+    const void* map;      // TMA maps of G (forward, backward; 128 bytes each)
+    int s, u, ndOff, pad;
+};
+
+// One tile: rows row0 .. of front `front`, columns col0 .., K range [k0, ke)
+// in nst stages (and `carry` chunks of the children's updates of its update
+// rows); split `split` of `nsplit`.  It may start once done[dep0] >= need0 and
+// done[dep1] >= need1 (-1: no such dependency) and adds one to done[signal]
+// when its output is written.
+struct alignas(16) FlowTile {
+    int front, row0, col0, k0;
+    int ke, nst, dep0, need0;
+    int dep1, need1, signal, slot;
+    int counter;
+    short split, nsplit, carry, bwd;
+    int pad;
+};
+
+struct FlowWork {
+    void* rnd;       // [nSub][k] the panel's right-hand sides
+    void* w;         // [nSub][k] inv(D) Y
+    void* x;         // [nSub][k] solution
+    void* partials;  // split-K partial tiles
+    int* counters;   // arrivals of split tiles (zero between launches)
+    int* done;       // finished tiles per front, forward then backward (zero between launches)
+    int* ctrl;       // ticket, finished CTAs (zero between launches)
+    int* status;     // bit 2: a wait timed out
+    int numDone;
+};
+
+// Columns of a tile for k right-hand sides: the power of two that holds them, at most kFlowMaxCols.
+int FlowCols(int k);
+template <typename R>
+int FlowCarryChunks(int cols);
+// CTAs that run at once.
+int FlowSlots();
+template <typename R>
+void PrepareFlowKernels();
+// The two TMA maps (256 bytes, 64-byte aligned host memory) of a front's factor.
+template <typename R>
+void EncodeFlowMaps(const cpx<R>* G, int s, int u, int ldg, void* out);
+template <typename R>
+void LaunchFlowGather(const z64* B, cpx<R>* rnd, int nSub, int k, const PanelIO& io, cudaStream_t st);
+template <typename R>
+void LaunchFlow(const FlowFront<R>* fr, const FlowTile* tiles, int n, int k, z64* B, const PanelIO& io,
+                const FlowWork& w, cudaStream_t st);
+// The same tile list on the tensor cores (sweep_flow_tc.cu; complex single,
+// `cols` 16 or 32 right-hand sides per tile).
+void PrepareFlowTcKernels();
+int FlowTcSlots();
+void LaunchFlowTc(const FlowFront<float>* fr, const FlowTile* tiles, int n, int k, int cols, z64* B, const PanelIO& io,
+                  const FlowWork& w, cudaStream_t st);
 
 // ------------------------------------------------------------------ GMRES vectors
 

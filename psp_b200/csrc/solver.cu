@@ -10,8 +10,6 @@
 #include <cstring>
 #include <iostream>
 #include <limits>
-#include <map>
-#include <mutex>
 #include <string>
 #include <type_traits>
 
@@ -47,13 +45,6 @@ void TaskArena::Upload(cudaStream_t st) {
 namespace {
 
 typedef std::complex<double> Cd;
-
-// Sweep variants (kernel and K-chunk per depth) chosen by timing, shared by
-// every handle of the process with the same front structure, block width
-// and device: equal problems then run the same kernels (a re-initialized handle and a fresh
-// one give identical results) and a batch of equal problems is timed once.
-std::mutex gRouteMutex, gTuneMutex;
-std::map<std::string, std::vector<int>> gRoutes;
 
 // Imaginary stretch of a PML point at distance `delta` from the inner edge
 // (the common body of s1Inv/s2Inv/s3Inv/s3InvArtificial,
@@ -151,12 +142,13 @@ template <typename R>
 class FactorStore {
 public:
     explicit FactorStore(Helmholtz& h) : h_(h), an_(h.an_) {
-        PrepareSweepKernels<R>();
-        // Complex-single factors use the tensor-core sweep unless the
-        // environment asks for the CUDA-core kernels (for comparisons).
+        PrepareFlowKernels<R>();
+        // Complex-single factors use the tensor-core sweep from
+        // kFlowTcMinCols right-hand sides on, unless the environment asks for
+        // the CUDA cores (for comparisons).
         const char* env = std::getenv("PSP_B200_SWEEP_CUDA_CORES");
         tc_ = std::is_same<R, float>::value && !(env && env[0] == '1');
-        if (tc_) PrepareSweepTcKernels();
+        if (tc_) PrepareFlowTcKernels();
         // Likewise the factorization GEMMs of complex-single fronts.
         const char* fenv = std::getenv("PSP_B200_FACTOR_CUDA_CORES");
         factorTc_ = std::is_same<R, float>::value && !(fenv && fenv[0] == '1');
@@ -269,60 +261,29 @@ private:
     }
     std::vector<std::vector<int>> depthNodes_;
     DeviceBuffer status_;
-    // One way to run the solve GEMM of one depth and direction: the kernel
-    // (tensor cores, tiles of kTcRows rows; or CUDA cores, kSweepRows rows)
-    // and the K-chunk of its tiles.
-    struct SweepVariant {
-        bool tc = false;
-        int cols = kSweepCols;  // right-hand sides per tile (tensor cores: 16 or 32)
-        int chunk = 0;
-        size_t tiles = 0;  // arena offset of the tile list
-        int n = 0;
-    };
-    // Per tree depth and direction: the candidate variants and the one in
-    // use (complex single: chosen by timing them all, Autotune).
-    struct ClassPlan {
-        size_t pre = 0;
-        int preN = 0;
-        std::vector<size_t> bGather;
-        std::vector<int> bGatherN;
-        std::vector<std::vector<SweepVariant>> fVar, bVar;
-        std::vector<int> fSel, bSel;
-        std::vector<double> fFlops, fBytes, bFlops, bBytes;
-        const SweepVariant& F(int d) const { return fVar[d][fSel[d]]; }
-        const SweepVariant& B(int d) const { return bVar[d][bSel[d]]; }
-    };
     // Task lists and work vectors of the panel solves for one RHS block width.
     // Plans live as long as the factors: captured sweep graphs point into them.
     struct SolvePlan {
         int k = 0;
-        DeviceBuffer Rb, Y, Z, Xnd, partials, counters;
+        bool tc = false;  // on the tensor cores
+        int cols = 0;     // right-hand sides per tile
+        DeviceBuffer rnd, W, X, planes, partials, counters, done;
+        int planesClass = -1;  // class whose unwritten plane rows are zero
         TaskArena arena;
-        ClassPlan cplan[3];
+        // per class the ordered tile list (arena offset) and its work, per
+        // panel its fronts
+        size_t tiles[3] = {0, 0, 0};
+        int numTiles[3] = {0, 0, 0};
+        double flops[3] = {0, 0, 0}, bytes[3] = {0, 0, 0};
         std::vector<size_t> panelFronts;
-        // complex single: the tensor-core sweep's TMA maps, two per front
-        struct alignas(64) MapPair { unsigned char b[kSweepTcMapBytes]; };
+        // the TMA maps of the factors, two per front
+        struct alignas(64) MapPair { unsigned char b[kFlowMapBytes]; };
         std::vector<MapPair> mapsHost;
         DeviceBuffer maps;
     };
     std::vector<std::unique_ptr<SolvePlan>> plans_;
     SolvePlan& Plan(int k);
-    // Times every candidate variant of every depth of one panel solve per
-    // class (scratch right-hand sides; without room for them the default
-    // tiling stays) and keeps the fastest per depth and direction.  Events
-    // bracket each solve-GEMM launch while tune_ is set.
-    // Returns false when it measured nothing (no room for its scratch).
-    bool Autotune(SolvePlan& P);
-    struct TuneEvents {
-        std::vector<cudaEvent_t> ev;
-        int used = 0;
-    };
-    TuneEvents* tune_ = nullptr;
-    void TuneMark() {
-        if (tune_ && tune_->used < (int)tune_->ev.size())
-            CUDA_CHECK(cudaEventRecord(tune_->ev[tune_->used++], h_.stream_));
-    }
-    bool tc_ = false;  // tensor-core sweep kernels (complex single only)
+    bool tc_ = false;  // tensor-core sweep kernel (complex single only)
     bool factorTc_ = false;  // tensor-core factorization GEMMs (complex single only)
     // Ops of at least this many rows and K columns take tensor-core tiles.
     bool UseGemmTc(const GemmOp<R>& op) const { return factorTc_ && op.M >= 64 && op.K >= 16; }
@@ -842,382 +803,215 @@ void FactorStore<R>::RunProgram(FactorProgram& pg, bool sync) {
     if (sync) CUDA_CHECK(cudaStreamSynchronize(st));
 }
 
+// The work vectors, fronts and tile list of the panel solves for k right-hand
+// sides (sweep_flow.cu, sweep_flow_tc.cu).
 template <typename R>
 typename FactorStore<R>::SolvePlan& FactorStore<R>::Plan(int k) {
     for (auto& pl : plans_)
         if (pl->k == k) return *pl;
-    plans_.emplace_back(new SolvePlan);
-    SolvePlan& P = *plans_.back();
+    std::unique_ptr<SolvePlan> plan(new SolvePlan);
+    SolvePlan& P = *plan;
     P.k = k;
     const PanelGeometry& g = an_.geom;
     const XYTree& tree = an_.tree;
-    const int np = g.numPanels;
-    const int nd = (int)depthNodes_.size();
-    // Work vectors per class: R planes (3 (s+u) k), Y (s k) and Z ((s+u) k).
-    std::vector<std::vector<int64_t>> rOff(3), yOff(3), zOff(3);
-    int64_t maxR = 0, maxY = 0, maxZ = 0;
+    const int np = g.numPanels, nd = (int)depthNodes_.size();
+    constexpr int TR = FlowRows<R>();
+    P.tc = tc_ && k >= kFlowTcMinCols;
+    const int nc = P.cols = P.tc ? (k > 16 ? 32 : 16) : FlowCols(k);
+    const int carryChunks = P.tc ? 1 : FlowCarryChunks<R>(nc);
+    const int running = P.tc ? FlowTcSlots() : FlowSlots();  // CTAs that run at once
+    // per front two planes of s + u rows, one per child
     int maxSub = 0;
+    int64_t maxRows = 0;
+    std::vector<int64_t> planeOff[3];
     for (int c = 0; c < 3; ++c) {
         if (!an_.classUsed[c]) continue;
-        const ClassStructure& cs = an_.cls[c];
-        rOff[c].resize(nn_); yOff[c].resize(nn_); zOff[c].resize(nn_);
-        int64_t tr = 0, ty = 0, tz = 0;
+        maxSub = std::max(maxSub, an_.cls[c].nSub);
+        planeOff[c].assign(nn_, 0);
+        int64_t rows = 0;
         for (int t = 0; t < nn_; ++t) {
-            rOff[c][t] = tr; yOff[c][t] = ty; zOff[c][t] = tz;
-            tr += (int64_t)(cs.size[t] + cs.usize[t]) * 3 * k;
-            ty += (int64_t)cs.size[t] * k;
-            tz += (int64_t)(cs.size[t] + cs.usize[t]) * k;
+            planeOff[c][t] = rows;
+            if (tree.nodes[t].numChildren > 0) rows += 2 * (int64_t)(an_.cls[c].size[t] + an_.cls[c].usize[t]);
         }
-        maxR = std::max(maxR, tr); maxY = std::max(maxY, ty); maxZ = std::max(maxZ, tz);
-        maxSub = std::max(maxSub, cs.nSub);
+        maxRows = std::max(maxRows, rows);
     }
-    P.Rb.Allocate(maxR * sizeof(cpx<R>));
-    P.Y.Allocate(maxY * sizeof(cpx<R>));
-    P.Z.Allocate(maxZ * sizeof(cpx<R>));
-    P.Xnd.Allocate((size_t)maxSub * k * sizeof(cpx<R>));
+    P.rnd.Allocate((size_t)maxSub * k * sizeof(cpx<R>));
+    P.W.Allocate((size_t)maxSub * k * sizeof(cpx<R>));
+    P.X.Allocate((size_t)maxSub * k * sizeof(cpx<R>));
+    P.planes.Allocate((size_t)maxRows * k * sizeof(cpx<R>));
+    P.planesClass = -1;
     P.arena.host.clear();
     P.panelFronts.assign(np, 0);
-    if (tc_) {
-        P.mapsHost.assign((size_t)np * nn_, {});
-        P.maps.Allocate(P.mapsHost.size() * sizeof(typename SolvePlan::MapPair));
-    }
+    P.mapsHost.assign((size_t)np * nn_, {});
+    P.maps.Allocate(P.mapsHost.size() * sizeof(typename SolvePlan::MapPair));
     for (int p = 0; p < np; ++p) {
         const int c = g.Class(p);
         const ClassStructure& cs = an_.cls[c];
-        std::vector<SweepFront<R>> fr(nn_);
+        std::vector<FlowFront<R>> fr(nn_);
         for (int t = 0; t < nn_; ++t) {
-            SweepFront<R>& f = fr[t];
+            FlowFront<R>& f = fr[t];
+            std::memset(&f, 0, sizeof(f));
             const XYNode& node = tree.nodes[t];
-            f.G = gPtr_[(size_t)p * nn_ + t];
             f.D = dPtr_[(size_t)p * nn_ + t];
-            f.Rb = P.Rb.template as<cpx<R>>() + rOff[c][t];
-            f.parentRb = node.parent >= 0 ? P.Rb.template as<cpx<R>>() + rOff[c][node.parent] : nullptr;
-            f.Y = P.Y.template as<cpx<R>>() + yOff[c][t];
-            f.Z = P.Z.template as<cpx<R>>() + zOff[c][t];
-            f.lower = h_.dLower_[c].as<int>() + cs.lowerOff[t];
-            f.rel = h_.dRel_[c].as<int>() + cs.lowerOff[t];
+            cpx<R>* planes = P.planes.template as<cpx<R>>();
             f.s = cs.size[t];
             f.u = cs.usize[t];
             f.ndOff = cs.off[t];
-            f.childSlot = (node.parent >= 0 && tree.nodes[node.parent].child[1] == t) ? 1 : 0;
-            f.ldg = GLeadingDim(f.s, f.u);
-            f.tmap = nullptr;
-            if constexpr (std::is_same<R, float>::value) {
-                if (tc_ && f.s > 0 && owned_[p]) {
-                    const size_t i = (size_t)p * nn_ + t;
-                    EncodeSweepTcMaps(f, P.mapsHost[i].b);
-                    f.tmap = P.maps.template as<unsigned char>() + i * sizeof(typename SolvePlan::MapPair);
-                }
+            f.lower = h_.dLower_[c].as<int>() + cs.lowerOff[t];
+            f.rel = h_.dRel_[c].as<int>() + cs.lowerOff[t];
+            auto plane = [&](int node, int slot) {
+                return planes + (planeOff[c][node] + slot * (int64_t)(cs.size[node] + cs.usize[node])) * k;
+            };
+            if (node.parent >= 0) f.Pp = plane(node.parent, tree.nodes[node.parent].child[1] == t ? 1 : 0);
+            if (node.numChildren > 0 && cs.size[node.child[0]] > 0) f.P0 = plane(t, 0);
+            if (node.numChildren > 1 && cs.size[node.child[1]] > 0) f.P1 = plane(t, 1);
+            if (f.s > 0 && owned_[p]) {
+                const size_t i = (size_t)p * nn_ + t;
+                EncodeFlowMaps<R>(gPtr_[i], f.s, f.u, GLeadingDim(f.s, f.u), P.mapsHost[i].b);
+                f.map = P.maps.template as<unsigned char>() + i * sizeof(typename SolvePlan::MapPair);
             }
         }
         P.panelFronts[p] = P.arena.Push(fr);
     }
-    // Tiles of one depth and direction: rows of a tile share one K range
-    // (inv(L11) is triangular, so the forward range stops at the tile's last
-    // row and the backward range starts at its first), split into chunks.
-    // The default chunk starts at the kernel's longest (the tensor-core
-    // kernels are persistent and pipeline across tiles, so long chunks cost
-    // nothing extra and save split-K partial sums) and only shrinks to give
-    // every SM tiles; `forceChunk` > 0 fixes it instead (tuning candidates).
-    int64_t maxPartialRows = kTcRows, maxCounters = 1;
-    // Longest K-chunk of a tensor-core tile (PSP_B200_SWEEP_TC_MAX_CHUNK),
-    // and a fixed chunk for the default tensor-core tiling in place of the
-    // shrinking rule below (PSP_B200_SWEEP_TC_CHUNK, tests; 0 = unset).
-    // Both are rounded down to a power of two from 16 to 512: a backward
-    // tile's K start is the innermost coordinate of its TMA copies, which
-    // must be even (16-byte aligned complex-single entries), and chunks of
-    // whole stages keep it so.
+    // What a tile costs beside its stages, in stages (a stage takes about 0.4 us
+    // of a tensor-core CTA and 0.5 us of a CUDA-core one): its first right-hand
+    // sides and its write-out; when split, the exchange and the sum of the
+    // partials.  Measured from the tiles' time stamps; a sweep's time changes by
+    // 1 % when they are halved or doubled, but by 8 % (FP64, 57 x 53 x 61, k = 5:
+    // 7.4 ms instead of 6.9) when tiles of fewer than kMinStages are allowed.
+    constexpr int kMinStages = 8;
+    const double kTileCost = P.tc ? 4 : 6, kSplitCost = P.tc ? 4 : 2, kPartCost = P.tc ? 1.2 * nc / 16 : 0.2;
+    // The environment may fix the tensor-core tiles' K-chunk (tests compare
+    // chunk lengths) or bound it; rounded down to a power of two from 16 to 512.
     auto chunkSetting = [](long long v) {
-        int c = 16;
+        int c = kFlowStageK;
         while (2LL * c <= std::min(v, 512LL)) c *= 2;
-        return c;
+        return c / kFlowStageK;
     };
-    const int tcMaxChunk = chunkSetting(EnvInt("PSP_B200_SWEEP_TC_MAX_CHUNK", 512));
-    const long long tcChunkEnv = EnvInt("PSP_B200_SWEEP_TC_CHUNK", 0);
-    const int tcFixedChunk = tcChunkEnv > 0 ? std::min(tcMaxChunk, chunkSetting(tcChunkEnv)) : 0;
-    auto makeTiles = [&](const ClassStructure& cs, int d, bool fwd, bool tcTiles, int cols, int forceChunk,
-                         std::vector<SweepTile>& tiles) {
-        const int maxChunk = tcTiles ? tcMaxChunk : SweepMaxChunk<R>();
-        if (forceChunk > maxChunk) forceChunk = maxChunk;
-        const int tileRows = tcTiles ? kTcRows : kSweepRows;
-        const int subs = cols / kSweepCols;  // partial slots and counters per split tile
-        auto build = [&](int kc, bool emit) {
-            int64_t n = 0, slots = 0, counters = 0;
-            for (int t : depthNodes_[d]) {
-                const int s = cs.size[t], u = cs.usize[t];
-                const int M = fwd ? s + u : s, K = fwd ? s : s + u;
-                for (int col0 = 0; col0 < k; col0 += cols)
-                    for (int row0 = 0; row0 < M; row0 += tileRows) {
-                        const int kb = fwd ? 0 : row0;
-                        const int ke = fwd ? std::min(K, row0 + tileRows) : K;
-                        const int ns = std::max(1, (int)CeilDiv(ke - kb, kc));
-                        for (int sp = 0; sp < ns; ++sp) {
-                            if (emit) {
-                                SweepTile tl;
-                                tl.front = t; tl.row0 = row0; tl.col0 = col0;
-                                tl.k0 = kb + sp * kc;
-                                tl.k1 = std::min(ke, kb + (sp + 1) * kc);
-                                tl.split = sp; tl.nsplit = ns;
-                                tl.slot = ns > 1 ? (int)slots : -1;
-                                tl.counter = ns > 1 ? (int)counters : -1;
-                                tiles.push_back(tl);
-                            }
-                            ++n;
-                        }
-                        if (ns > 1) { slots += ns; ++counters; }
-                    }
-            }
-            if (emit) {
-                maxPartialRows = std::max(maxPartialRows, slots * tileRows * subs);
-                maxCounters = std::max(maxCounters, counters * subs);
-            }
-            return n;
-        };
-        // default: shrink until the launch has tiles for every SM (CUDA-core
-        // CTAs, two per SM) or for half of them (persistent tensor-core CTAs,
-        // whose long K pipelines beat extra split-K partial sums)
-        const int64_t minTiles = tcTiles ? 74 : 2 * 148;
-        int kc = forceChunk > 0 ? forceChunk : maxChunk;
-        while (forceChunk <= 0 && kc > 64 && build(kc, false) < minTiles) kc /= 2;
-        build(kc, true);
-        // longest K ranges first, so the launch does not end on a long tail
-        std::stable_sort(tiles.begin(), tiles.end(), [](const SweepTile& a, const SweepTile& b) {
-            return (a.k1 - a.k0) > (b.k1 - b.k0);
-        });
-        return kc;
-    };
-    auto depthCost = [&](const ClassStructure& cs, int d, bool fwd, double& flops, double& bytes) {
-        for (int t : depthNodes_[d]) {
-            const double s = cs.size[t], u = cs.usize[t];
-            const double nz = (s + u) * s - s * (s - 1) / 2;  // nonzeros of G
-            flops += 8.0 * nz * k;
-            bytes += sizeof(cpx<R>) * (nz + (fwd ? (s + 2 * (s + u)) : (2 * (s + u) + 2 * s)) * k);
-        }
-    };
-    // Candidates of one depth and direction: the default tiling of each
-    // kernel and, with tensor cores, the other chunk lengths (a tiling equal
-    // to an earlier candidate's is skipped).
-    // With more than 16 right-hand sides the tensor-core tiles take 32 of
-    // them (one split of each G stage for twice the columns); the 16-wide
-    // default stays a candidate.
-    auto makeVariants = [&](const ClassStructure& cs, int d, bool fwd, std::vector<SweepVariant>& out) {
-        struct Cand { bool tc; int cols, chunk; };
-        std::vector<Cand> cand;
-        if (tc_) {
-            const int wide = k > kSweepCols ? 32 : kSweepCols;
-            cand.push_back({true, wide, tcFixedChunk});
-            for (int kc : {64, 128, 256, 512}) cand.push_back({true, wide, kc});
-            if (wide != kSweepCols)
-                for (int kc : {0, 512}) cand.push_back({true, kSweepCols, kc});
-            cand.push_back({false, kSweepCols, 0});
-            for (int kc : {64, 128}) cand.push_back({false, kSweepCols, kc});
-        } else {
-            cand.push_back({false, kSweepCols, 0});
-        }
-        std::vector<std::vector<SweepTile>> seen;
-        for (const auto& cd : cand) {
-            std::vector<SweepTile> tiles;
-            SweepVariant v;
-            v.tc = cd.tc;
-            v.cols = cd.cols;
-            v.chunk = makeTiles(cs, d, fwd, cd.tc, cd.cols, cd.chunk, tiles);
-            bool dup = false;
-            for (size_t i = 0; i < seen.size() && !dup; ++i)
-                dup = out[i].tc == v.tc && out[i].cols == v.cols && seen[i].size() == tiles.size() &&
-                      std::equal(tiles.begin(), tiles.end(), seen[i].begin(), [](const SweepTile& a, const SweepTile& b) {
-                          return a.front == b.front && a.row0 == b.row0 && a.col0 == b.col0 && a.k0 == b.k0 &&
-                                 a.k1 == b.k1;
-                      });
-            if (dup) continue;
-            v.tiles = P.arena.Push(tiles);
-            v.n = (int)tiles.size();
-            out.push_back(v);
-            seen.push_back(std::move(tiles));
-        }
-    };
+    const long long fixedEnv = P.tc ? EnvInt("PSP_B200_SWEEP_TC_CHUNK", 0) : 0;
+    const long long maxEnv = P.tc ? EnvInt("PSP_B200_SWEEP_TC_MAX_CHUNK", 0) : 0;
+    int64_t maxSlots = 1, maxCounters = 1;
     for (int c = 0; c < 3; ++c) {
         if (!an_.classUsed[c]) continue;
         const ClassStructure& cs = an_.cls[c];
-        ClassPlan& cp = P.cplan[c];
-        cp.bGather.assign(nd, 0);
-        cp.bGatherN.assign(nd, 0);
-        cp.fVar.assign(nd, {});
-        cp.bVar.assign(nd, {});
-        cp.fSel.assign(nd, 0);
-        cp.bSel.assign(nd, 0);
-        cp.fFlops.assign(nd, 0); cp.fBytes.assign(nd, 0); cp.bFlops.assign(nd, 0); cp.bBytes.assign(nd, 0);
-        std::vector<int2> pre;
-        for (int d = 0; d < nd; ++d) {
-            std::vector<int2> bg;
-            makeVariants(cs, d, true, cp.fVar[d]);
-            makeVariants(cs, d, false, cp.bVar[d]);
-            depthCost(cs, d, true, cp.fFlops[d], cp.fBytes[d]);
-            depthCost(cs, d, false, cp.bFlops[d], cp.bBytes[d]);
-            for (int t : depthNodes_[d])
-                for (int i0 = 0; i0 < cs.size[t] + cs.usize[t]; i0 += kSweepRows) {
-                    bg.push_back(make_int2(t, i0));
-                    pre.push_back(make_int2(t, i0));
-                }
-            cp.bGather[d] = P.arena.Push(bg);
-            cp.bGatherN[d] = (int)bg.size();
-        }
-        cp.pre = P.arena.Push(pre);
-        cp.preN = (int)pre.size();
-    }
-    P.partials.Allocate((size_t)maxPartialRows * kSweepCols * sizeof(cpx<R>));
-    P.counters.Allocate((size_t)maxCounters * sizeof(int));
-    CUDA_CHECK(cudaMemsetAsync(P.counters.p, 0, P.counters.bytes, h_.stream_));
-    P.arena.Upload(h_.stream_);
-    if (tc_) {
-        CUDA_CHECK(cudaMemcpyAsync(P.maps.p, P.mapsHost.data(), P.maps.bytes, cudaMemcpyHostToDevice, h_.stream_));
-        // PSP_B200_SWEEP_AUTOTUNE: unset = time every candidate per depth on
-        // problems of at least 2^20 unknowns (where the timing, a few sweeps'
-        // worth, is small against a solve), else the default tiling; "1" =
-        // time them at any size; "0" = the default tensor-core tiling
-        // everywhere; "alternate" = a fixed mix of tensor-core and CUDA-core
-        // depths (tests).
-        const char* env = std::getenv("PSP_B200_SWEEP_AUTOTUNE");
-        std::string mode = env ? env : "";
-        if (mode.empty()) mode = h_.NumUnknowns() >= (int64_t(1) << 20) ? "1" : "0";
-        if (mode == "alternate") {
-            for (ClassPlan& cp : P.cplan)
-                for (size_t d = 0; d < cp.fVar.size(); ++d) {
-                    auto firstOf = [](const std::vector<SweepVariant>& vs, bool tc) {
-                        for (size_t i = 0; i < vs.size(); ++i)
-                            if (vs[i].tc == tc) return (int)i;
-                        return 0;
-                    };
-                    cp.fSel[d] = firstOf(cp.fVar[d], d % 2 == 1);
-                    cp.bSel[d] = firstOf(cp.bVar[d], d % 2 == 0);
-                }
-        } else if (mode == "1") {
-            std::string key = std::to_string(k) + "/" + std::to_string(h_.device());
-            for (int c = 0; c < 3; ++c) {
-                if (!an_.classUsed[c]) continue;
-                const ClassStructure& cs = an_.cls[c];
-                key += "|" + std::to_string(c) + ":";
-                for (size_t t = 0; t < cs.size.size(); ++t)
-                    key += std::to_string(cs.size[t]) + "," + std::to_string(cs.usize[t]) + ";";
-            }
-            std::vector<int> routes;
-            auto lookup = [&] {
-                std::lock_guard<std::mutex> lock(gRouteMutex);
-                auto it = gRoutes.find(key);
-                if (it != gRoutes.end()) routes = it->second;
+        std::vector<FlowTile> list;
+        const int colTiles = (int)CeilDiv(k, nc);
+        auto outputs = [&](int t, bool fwd) {
+            return (int)CeilDiv(fwd ? cs.size[t] + cs.usize[t] : cs.size[t], TR) * colTiles;
+        };
+        int64_t slots = 0, counters = 0;
+        for (int ph = 0; ph < 2 * nd; ++ph) {
+            const bool fwd = ph < nd;
+            const int d = fwd ? nd - 1 - ph : ph - nd;
+            if (ph == nd) { maxSlots = std::max(maxSlots, slots); slots = 0; }  // backward starts after all of forward
+            // K range of a row tile (inv(L11) is triangular)
+            auto range = [&](int t, int row0, int& kb, int& ke) {
+                const int s = cs.size[t], u = cs.usize[t];
+                kb = fwd ? 0 : row0;
+                ke = fwd ? std::min(s, row0 + TR) : s + u;
             };
-            lookup();
-            if (routes.empty()) {
-                // one tuning run at a time in the process: a handle with the
-                // same structure waits for it and reuses its choices, and
-                // no two tuning runs time each other's launches
-                std::lock_guard<std::mutex> tuning(gTuneMutex);
-                lookup();
-                if (routes.empty() && Autotune(P)) {
-                    // only measured choices are shared: a handle that could
-                    // not time its candidates keeps the default tiling, and a
-                    // later one with room tunes
-                    for (const ClassPlan& cp : P.cplan) {
-                        routes.insert(routes.end(), cp.fSel.begin(), cp.fSel.end());
-                        routes.insert(routes.end(), cp.bSel.begin(), cp.bSel.end());
-                    }
-                    std::lock_guard<std::mutex> lock(gRouteMutex);
-                    gRoutes.emplace(key, routes);
+            // The longest tile (stages): of the candidates, the one whose tiles
+            // take least when the CTAs that run at once share them.
+            std::vector<int> work;  // stages of every row tile
+            for (int t : depthNodes_[d]) {
+                if (cs.size[t] == 0) continue;
+                const int M = fwd ? cs.size[t] + cs.usize[t] : cs.size[t];
+                for (int row0 = 0; row0 < M; row0 += TR) {
+                    int kb, ke;
+                    range(t, row0, kb, ke);
+                    for (int ct = 0; ct < colTiles; ++ct) work.push_back((int)CeilDiv(ke - kb, kFlowStageK));
                 }
             }
-            size_t i = 0;
-            for (ClassPlan& cp : P.cplan) {
-                for (int& r : cp.fSel) r = routes.empty() ? 0 : routes[i++];
-                for (int& r : cp.bSel) r = routes.empty() ? 0 : routes[i++];
+            int chunk = 1 << 20;
+            double best = 1e30;
+            for (int cand : {kMinStages, 10, 12, 16, 20, 24, 32, 48, 64, 1 << 20}) {
+                double total = 0, longest = 0;
+                size_t count = 0;
+                for (int nst : work) {
+                    const int ns = (int)CeilDiv(nst, cand), per = (int)CeilDiv(nst, ns), parts = (int)CeilDiv(nst, per);
+                    const double cost = kTileCost + per + (parts > 1 ? kSplitCost + kPartCost * parts : 0);
+                    total += cost * parts;
+                    longest = std::max(longest, cost);
+                    count += parts;
+                }
+                // rounds of equal tiles over the CTAs, or an even share of the work
+                const double span = std::max({longest, total / running, longest * CeilDiv((int64_t)count, running) * 0.85});
+                if (span < best) { best = span; chunk = cand; }
             }
+            if (fixedEnv > 0) chunk = chunkSetting(fixedEnv);
+            if (maxEnv > 0) chunk = std::min(chunk, chunkSetting(maxEnv));
+            const size_t first = list.size();
+            for (int t : depthNodes_[d]) {
+                const int s = cs.size[t], u = cs.usize[t];
+                if (s == 0) continue;
+                const XYNode& node = tree.nodes[t];
+                const int M = fwd ? s + u : s;
+                for (int col0 = 0; col0 < k; col0 += nc)
+                    for (int row0 = 0; row0 < M; row0 += TR) {
+                        int kb, ke;
+                        range(t, row0, kb, ke);
+                        const int nst = (int)CeilDiv(ke - kb, kFlowStageK);
+                        const int ns = (int)CeilDiv(nst, chunk), per = (int)CeilDiv(nst, ns);
+                        FlowTile tl;
+                        std::memset(&tl, 0, sizeof(tl));
+                        tl.front = t; tl.row0 = row0; tl.col0 = col0;
+                        tl.dep0 = tl.dep1 = -1;
+                        tl.bwd = !fwd;
+                        tl.signal = fwd ? t : nn_ + t;
+                        if (fwd) {
+                            for (int slot = 0; slot < node.numChildren; ++slot) {
+                                const int ch = node.child[slot];
+                                if (cs.size[ch] == 0) continue;
+                                (slot ? tl.dep1 : tl.dep0) = ch;
+                                (slot ? tl.need1 : tl.need0) = outputs(ch, true);
+                            }
+                        } else if (node.parent >= 0) {
+                            tl.dep0 = nn_ + node.parent;
+                            tl.need0 = outputs(node.parent, false);
+                        } else {
+                            tl.dep0 = t;
+                            tl.need0 = outputs(t, true);
+                        }
+                        const int parts = (int)CeilDiv(nst, per);
+                        for (int sp = 0; sp < parts; ++sp) {
+                            tl.k0 = kb + sp * per * kFlowStageK;
+                            tl.ke = std::min(ke, tl.k0 + per * kFlowStageK);
+                            tl.nst = (int)CeilDiv(tl.ke - tl.k0, kFlowStageK);
+                            tl.split = (short)sp;
+                            tl.nsplit = (short)parts;
+                            tl.slot = parts > 1 ? (int)slots : -1;
+                            tl.counter = parts > 1 ? (int)counters : -1;
+                            tl.carry = (short)(fwd && sp == 0 && row0 + TR > s && u > 0 && node.numChildren > 0 ? carryChunks : 0);
+                            list.push_back(tl);
+                        }
+                        if (parts > 1) { slots += parts; ++counters; }
+                    }
+            }
+            // longest first, so the phase does not end on a long tile
+            std::stable_sort(list.begin() + first, list.end(),
+                             [](const FlowTile& a, const FlowTile& b) { return a.nst + a.carry > b.nst + b.carry; });
+        }
+        maxSlots = std::max(maxSlots, slots);
+        maxCounters = std::max(maxCounters, counters);
+        P.numTiles[c] = (int)list.size();
+        P.tiles[c] = P.arena.Push(list);
+        for (int t = 0; t < nn_; ++t) {
+            const double s = cs.size[t], u = cs.usize[t];
+            const double nz = (s + u) * s - s * (s - 1) / 2;  // nonzeros of G
+            P.flops[c] += 2 * 8.0 * nz * k;
+            P.bytes[c] += sizeof(cpx<R>) * (2 * nz + (s + 2 * (s + u) + 2 * (s + u) + 2 * s) * k);
         }
     }
+    P.partials.Allocate((size_t)maxSlots * TR * nc * sizeof(cpx<R>));
+    P.counters.Allocate((size_t)maxCounters * sizeof(int));
+    P.done.Allocate((2 * (size_t)nn_ + 2) * sizeof(int));
+    CUDA_CHECK(cudaMemsetAsync(P.counters.p, 0, P.counters.bytes, h_.stream_));
+    CUDA_CHECK(cudaMemsetAsync(P.done.p, 0, P.done.bytes, h_.stream_));
+    P.arena.Upload(h_.stream_);
+    CUDA_CHECK(cudaMemcpyAsync(P.maps.p, P.mapsHost.data(), P.maps.bytes, cudaMemcpyHostToDevice, h_.stream_));
+    CUDA_CHECK(cudaStreamSynchronize(h_.stream_));
+    plans_.push_back(std::move(plan));
     return P;
-}
-
-template <typename R>
-bool FactorStore<R>::Autotune(SolvePlan& P) {
-    const PanelGeometry& g = an_.geom;
-    const int nd = (int)depthNodes_.size(), k = P.k;
-    const int reps = 2;
-    DeviceBuffer scratch;
-    try {
-        scratch.Allocate((size_t)h_.NumUnknowns() * k * sizeof(z64));
-    } catch (const PspError& e) {
-        if (e.code != kOutOfMemory) throw;
-        cudaGetLastError();  // no room for timing runs: keep the default tiling
-        return false;
-    }
-    CUDA_CHECK(cudaMemsetAsync(scratch.p, 0, scratch.bytes, h_.stream_));
-    TuneEvents te;
-    te.ev.resize(4 * nd);
-    for (cudaEvent_t& e : te.ev) CUDA_CHECK(cudaEventCreate(&e));
-    const char* verbose = std::getenv("PSP_B200_SWEEP_AUTOTUNE_VERBOSE");
-    const bool talk = verbose && verbose[0] == '1';
-    try {
-        for (int c = 0; c < 3; ++c) {
-            int p = -1;
-            for (int q = 0; q < g.numPanels && p < 0; ++q)
-                if (g.Class(q) == c && owned_[q]) p = q;
-            if (p < 0) continue;
-            ClassPlan& cp = P.cplan[c];
-            size_t maxVar = 0;
-            for (int d = 0; d < nd; ++d) maxVar = std::max({maxVar, cp.fVar[d].size(), cp.bVar[d].size()});
-            // [direction][depth][variant] best milliseconds
-            std::vector<std::vector<float>> best[2];
-            for (int dir = 0; dir < 2; ++dir) {
-                best[dir].assign(nd, {});
-                for (int d = 0; d < nd; ++d) best[dir][d].assign((dir ? cp.bVar : cp.fVar)[d].size(), 1e30f);
-            }
-            // run v times every depth's v-th candidate (its first where it has fewer)
-            for (size_t v = 0; v < maxVar; ++v) {
-                for (int d = 0; d < nd; ++d) {
-                    cp.fSel[d] = v < cp.fVar[d].size() ? (int)v : 0;
-                    cp.bSel[d] = v < cp.bVar[d].size() ? (int)v : 0;
-                }
-                for (int rep = 0; rep <= reps; ++rep) {
-                    te.used = 0;
-                    tune_ = &te;
-                    SolvePanel(scratch.as<z64>(), k, k, p, 0, 0);
-                    tune_ = nullptr;
-                    CUDA_CHECK(cudaStreamSynchronize(h_.stream_));
-                    if (rep == 0 || te.used != 4 * nd) continue;  // the first run warms up
-                    for (int i = 0; i < nd; ++i) {
-                        float fms = 0, bms = 0;
-                        CUDA_CHECK(cudaEventElapsedTime(&fms, te.ev[2 * i], te.ev[2 * i + 1]));
-                        CUDA_CHECK(cudaEventElapsedTime(&bms, te.ev[2 * nd + 2 * i], te.ev[2 * nd + 2 * i + 1]));
-                        const int df = nd - 1 - i;  // the forward walks the depths bottom-up
-                        float& bf = best[0][df][cp.fSel[df]];
-                        float& bb = best[1][i][cp.bSel[i]];
-                        bf = std::min(bf, fms);
-                        bb = std::min(bb, bms);
-                    }
-                }
-            }
-            for (int d = 0; d < nd; ++d) {
-                for (int dir = 0; dir < 2; ++dir) {
-                    const std::vector<float>& b = best[dir][d];
-                    (dir ? cp.bSel : cp.fSel)[d] = (int)(std::min_element(b.begin(), b.end()) - b.begin());
-                }
-                if (talk) {
-                    std::fprintf(stderr, "sweep autotune k=%d class %d depth %2d:", k, c, d);
-                    for (int dir = 0; dir < 2; ++dir) {
-                        const std::vector<SweepVariant>& vs = (dir ? cp.bVar : cp.fVar)[d];
-                        std::fprintf(stderr, dir ? "  bwd" : " fwd");
-                        for (size_t i = 0; i < vs.size(); ++i)
-                            std::fprintf(stderr, " %s%s%d/%d %.4f", (int)i == (dir ? cp.bSel : cp.fSel)[d] ? "*" : "",
-                                         vs[i].tc ? "tc" : "cc", vs[i].cols, vs[i].chunk, best[dir][d][i]);
-                    }
-                    std::fprintf(stderr, "\n");
-                }
-            }
-        }
-    } catch (...) {
-        tune_ = nullptr;
-        for (cudaEvent_t e : te.ev) cudaEventDestroy(e);
-        throw;
-    }
-    for (cudaEvent_t e : te.ev) CUDA_CHECK(cudaEventDestroy(e));
-    return true;
 }
 
 template <typename R>
@@ -1227,7 +1021,6 @@ void FactorStore<R>::SolvePanel(z64* B, int ldk, int k, int p, int inMode, int o
     EnsurePanel(p);
     const PanelGeometry& g = an_.geom;
     const int c = g.Class(p);
-    const ClassPlan& cp = P.cplan[c];
     cudaStream_t st = h_.stream_;
     PanelIO io;
     io.ndToNat = h_.dNdToNat_[c].as<int>();
@@ -1242,52 +1035,34 @@ void FactorStore<R>::SolvePanel(z64* B, int ldk, int k, int p, int inMode, int o
     io.inMode = inMode;
     io.outAccumulate = outAcc;
     io.sp = h_.sp_;
-    const SweepFront<R>* fr = P.arena.template At<SweepFront<R>>(P.panelFronts[p]);
-    SweepWork w;
+    FlowWork w;
+    w.rnd = P.rnd.p;
+    w.w = P.W.p;
+    w.x = P.X.p;
     w.partials = P.partials.p;
     w.counters = P.counters.template as<int>();
-    w.xnd = P.Xnd.p;
+    w.ctrl = P.done.template as<int>();
+    w.done = w.ctrl + 2;
+    w.numDone = 2 * nn_;
     w.status = status_.template as<int>();
-    const int nd = (int)depthNodes_.size();
     {
         ProfScope ps(st, kProfGatherScatter);
-        LaunchSweepPregather<R>(fr, P.arena.template At<int2>(cp.pre), cp.preN, B, k, io, st, tc_);
-    }
-    for (int d = nd - 1; d >= 0; --d) {
-        ProfScope ps(st, kProfSolveGemm, cp.fFlops[d], cp.fBytes[d]);
-        const SweepVariant& v = cp.F(d);
-        const SweepTile* tl = P.arena.template At<SweepTile>(v.tiles);
-        TuneMark();
-        bool done = false;
-        if constexpr (std::is_same<R, float>::value) {
-            if (v.tc) {
-                LaunchSweepForwardTc(fr, tl, v.n, k, v.cols, w, st);
-                done = true;
-            }
+        if (P.planesClass != c) {
+            CUDA_CHECK(cudaMemsetAsync(P.planes.p, 0, P.planes.bytes, st));
+            P.planesClass = c;
         }
-        if (!done) LaunchSweepForward<R>(fr, tl, v.n, v.chunk, k, w, st);
-        TuneMark();
+        LaunchFlowGather<R>(B, P.rnd.template as<cpx<R>>(), an_.cls[c].nSub, k, io, st);
     }
-    for (int d = 0; d < nd; ++d) {
-        {
-            ProfScope ps(st, kProfGatherScatter);
-            LaunchSweepBackwardGather<R>(fr, P.arena.template At<int2>(cp.bGather[d]), cp.bGatherN[d], k, w, st,
-                                         cp.B(d).tc);
+    ProfScope ps(st, kProfSolveGemm, P.flops[c], P.bytes[c]);
+    const FlowFront<R>* fr = P.arena.template At<FlowFront<R>>(P.panelFronts[p]);
+    const FlowTile* tiles = P.arena.template At<FlowTile>(P.tiles[c]);
+    if constexpr (std::is_same<R, float>::value) {
+        if (P.tc) {
+            LaunchFlowTc(fr, tiles, P.numTiles[c], k, P.cols, B, io, w, st);
+            return;
         }
-        ProfScope ps(st, kProfSolveGemm, cp.bFlops[d], cp.bBytes[d]);
-        const SweepVariant& v = cp.B(d);
-        const SweepTile* tl = P.arena.template At<SweepTile>(v.tiles);
-        TuneMark();
-        bool done = false;
-        if constexpr (std::is_same<R, float>::value) {
-            if (v.tc) {
-                LaunchSweepBackwardTc(fr, tl, v.n, B, k, v.cols, io, w, st);
-                done = true;
-            }
-        }
-        if (!done) LaunchSweepBackward<R>(fr, tl, v.n, v.chunk, B, k, io, w, st);
-        TuneMark();
     }
+    LaunchFlow<R>(fr, tiles, P.numTiles[c], k, B, io, w, st);
 }
 
 template <typename R>
@@ -1308,10 +1083,11 @@ void FactorStore<R>::Sweep(z64* B, int ldk, int k, bool useGraph) {
         SweepEager(B, ldk, k);
         return;
     }
-    Plan(k);  // built outside the capture: it allocates and uploads
+    SolvePlan& P = Plan(k);  // built outside the capture: it allocates and uploads
     for (const SweepGraph& g : graphs_)
         if (g.B == B && g.ldk == ldk && g.k == k) {
             CUDA_CHECK(cudaGraphLaunch(g.exec, h_.stream_));
+            P.planesClass = an_.geom.Class(0);  // of the sweep's last panel solve
             return;
         }
     if (graphs_.size() >= 8) {  // graphs of earlier work vectors (the scratch moved)
@@ -1320,6 +1096,7 @@ void FactorStore<R>::Sweep(z64* B, int ldk, int k, bool useGraph) {
     }
     cudaGraph_t graph;
     CUDA_CHECK(cudaStreamBeginCapture(h_.stream_, cudaStreamCaptureModeThreadLocal));
+    P.planesClass = -1;  // the graph clears the planes whatever ran before it
     SweepEager(B, ldk, k);
     CUDA_CHECK(cudaStreamEndCapture(h_.stream_, &graph));
     SweepGraph g{B, ldk, k, nullptr};
@@ -1335,8 +1112,9 @@ double FactorStore<R>::PlanBytesPerRhs() const {
     for (int c = 0; c < 3; ++c) {
         if (!an_.classUsed[c]) continue;
         const ClassStructure& cs = an_.cls[c];
-        double e = cs.nSub;
-        for (size_t t = 0; t < cs.size.size(); ++t) e += 3.0 * (cs.size[t] + cs.usize[t]) + cs.size[t] + (cs.size[t] + cs.usize[t]);
+        double e = 3.0 * cs.nSub;
+        for (size_t t = 0; t < cs.size.size(); ++t)
+            if (an_.tree.nodes[t].numChildren > 0) e += 2.0 * (cs.size[t] + cs.usize[t]);
         best = std::max(best, e);
     }
     return best * sizeof(cpx<R>);

@@ -1,11 +1,7 @@
 // Minimal sm_100a tensor-core toolkit: tcgen05 MMA with operands in shared
 // memory and the accumulator in tensor memory (TMEM), completion through
 // mbarriers.  Layout and descriptor encodings follow the sm100 UMMA
-// definitions (SWIZZLE_NONE, K-major canonical layout):
-//   a K-major operand tile of R rows x K tf32 values is stored as 8-row x
-//   16-byte "core matrices" (rows 16 B apart); the K-chunks of one 8-row
-//   group are kChunkBytes apart (the descriptor's leading byte offset) and
-//   consecutive 8-row groups are sbo bytes apart (its stride byte offset).
+// definitions (K-major operands in the swizzled canonical layouts).
 #pragma once
 #include <cuda_runtime.h>
 
@@ -14,29 +10,8 @@
 namespace psp_b200 {
 namespace umma {
 
-constexpr uint32_t kChunkBytes = 128;  // one core matrix: 8 rows x 16 bytes
-
-// Byte offset of element (row, k) of a K-major tile whose 8-row groups are
-// `sbo` bytes apart.
-__device__ __forceinline__ uint32_t KMajorOffset(int row, int k, uint32_t sbo) {
-    return (uint32_t)(row >> 3) * sbo + (uint32_t)(k >> 2) * kChunkBytes + (uint32_t)(row & 7) * 16u +
-           (uint32_t)(k & 3) * 4u;
-}
-
 __device__ __forceinline__ uint32_t SmemAddr(const void* p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-
-// Shared-memory matrix descriptor: start address, leading byte offset (between
-// the two 16-byte K-chunks an MMA consumes), stride byte offset (between
-// 8-row groups), version 1, no swizzle.
-__device__ __forceinline__ uint64_t SmemDesc(uint32_t smemAddr, uint32_t lbo, uint32_t sbo) {
-    uint64_t d = 0;
-    d |= (uint64_t)((smemAddr >> 4) & 0x3FFF);
-    d |= (uint64_t)((lbo >> 4) & 0x3FFF) << 16;
-    d |= (uint64_t)((sbo >> 4) & 0x3FFF) << 32;
-    d |= (uint64_t)1 << 46;  // descriptor version for sm100
-    return d;
 }
 
 // Descriptor of a K-major operand in the 128-byte-swizzle layout: rows of
@@ -79,17 +54,7 @@ __host__ __device__ constexpr uint32_t InstrDescTf32(int M, int N) {
     return (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 
-__device__ __forceinline__ void MmaTf32(uint32_t tmemD, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                        uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}\n"
-        :
-        : "r"(tmemD), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate));
-}
-
-// The same with A read from tensor memory: M rows in TMEM lanes 0..M-1, one
+// D (+)= A B with A read from tensor memory: M rows in TMEM lanes 0..M-1, one
 // tf32 K value per 32-bit column starting at column address tmemA.
 __device__ __forceinline__ void MmaTf32TmemA(uint32_t tmemD, uint32_t tmemA, uint64_t bdesc, uint32_t idesc,
                                              uint32_t accumulate) {
@@ -201,33 +166,6 @@ __device__ __forceinline__ void CpAsyncWait() {
     asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 __device__ __forceinline__ void CpAsyncWaitAll() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-// Arrive on `mbar` once all prior cp.async copies of this thread have landed;
-// the arrival counts against the barrier's initial count.
-__device__ __forceinline__ void CpAsyncArrive(uint64_t* mbar) {
-    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(SmemAddr(mbar)) : "memory");
-}
-// Bulk asynchronous copy of `bytes` (a multiple of 16; both addresses 16-byte
-// aligned) from global to this CTA's shared memory, completing as
-// transaction bytes on `mbar`.
-__device__ __forceinline__ void BulkCopy(void* dst, const void* src, uint32_t bytes, uint64_t* mbar) {
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(SmemAddr(dst)),
-        "l"(src), "r"(bytes), "r"(SmemAddr(mbar))
-        : "memory");
-}
-// Tiled 2-D tensor copy (no multicast) of the box at coordinates (x, y) of
-// the tensor map at `tmap` (global memory, 64-byte aligned) into this CTA's
-// shared memory (128-byte aligned), completing as transaction bytes on
-// `mbar`; elements outside the tensor are zero-filled.  x * element size
-// must be a multiple of 16 bytes.
-__device__ __forceinline__ void TmaLoad2D(void* dst, const void* tmap, int x, int y, uint64_t* mbar) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], "
-        "[%4];" ::"r"(SmemAddr(dst)),
-        "l"(tmap), "r"(x), "r"(y), "r"(SmemAddr(mbar))
-        : "memory");
-}
-
 // Arrive on `mbar` and add `bytes` to the transaction bytes its phase waits for.
 __device__ __forceinline__ void MbarArriveExpectTx(uint64_t* mbar, uint32_t bytes) {
     asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1;\n\t}" ::"r"(
@@ -278,24 +216,17 @@ __device__ __forceinline__ void TmemStore32NoWait(uint32_t taddr, const float (&
         : "memory");
 }
 
-// Writes 32 consecutive f32 columns of this thread's TMEM lane and waits
-// for the write.
-__device__ __forceinline__ void TmemStore32(uint32_t taddr, const float (&v)[32]) {
+// Writes 16 consecutive 32-bit columns of this thread's TMEM lane without
+// waiting.
+__device__ __forceinline__ void TmemStore16(uint32_t taddr, const float (&v)[16]) {
     asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-        "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,"
-        "%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};\n"
-        ::"r"(taddr),
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};\n" ::"r"(
+            taddr),
         "r"(__float_as_uint(v[0])), "r"(__float_as_uint(v[1])), "r"(__float_as_uint(v[2])), "r"(__float_as_uint(v[3])),
         "r"(__float_as_uint(v[4])), "r"(__float_as_uint(v[5])), "r"(__float_as_uint(v[6])), "r"(__float_as_uint(v[7])),
         "r"(__float_as_uint(v[8])), "r"(__float_as_uint(v[9])), "r"(__float_as_uint(v[10])), "r"(__float_as_uint(v[11])),
-        "r"(__float_as_uint(v[12])), "r"(__float_as_uint(v[13])), "r"(__float_as_uint(v[14])), "r"(__float_as_uint(v[15])),
-        "r"(__float_as_uint(v[16])), "r"(__float_as_uint(v[17])), "r"(__float_as_uint(v[18])), "r"(__float_as_uint(v[19])),
-        "r"(__float_as_uint(v[20])), "r"(__float_as_uint(v[21])), "r"(__float_as_uint(v[22])), "r"(__float_as_uint(v[23])),
-        "r"(__float_as_uint(v[24])), "r"(__float_as_uint(v[25])), "r"(__float_as_uint(v[26])), "r"(__float_as_uint(v[27])),
-        "r"(__float_as_uint(v[28])), "r"(__float_as_uint(v[29])), "r"(__float_as_uint(v[30])), "r"(__float_as_uint(v[31]))
+        "r"(__float_as_uint(v[12])), "r"(__float_as_uint(v[13])), "r"(__float_as_uint(v[14])), "r"(__float_as_uint(v[15]))
         : "memory");
-    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 
 // Writes 8 consecutive 32-bit columns of this thread's TMEM lane without
@@ -330,16 +261,6 @@ __device__ __forceinline__ void TmemLoad16(uint32_t taddr, float (&v)[16]) {
 __device__ __forceinline__ void SplitTf32Fast(float x, float& hi, float& lo) {
     hi = __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xFFFFE000u);
     lo = x - hi;
-}
-
-// Split x into a tf32 head and a tf32 tail: x ~= hi + lo to ~2^-22 relative.
-__device__ __forceinline__ void SplitTf32(float x, float& hi, float& lo) {
-    uint32_t h;
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(h) : "f"(x));
-    hi = __uint_as_float(h);
-    uint32_t l;
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(l) : "f"(x - hi));
-    lo = __uint_as_float(l);
 }
 
 }  // namespace umma
