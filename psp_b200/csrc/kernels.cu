@@ -329,65 +329,107 @@ __global__ void __launch_bounds__(kThreads) ldl_trsm_kernel(const FactorFront<R>
 
 // ---------------------------------------------------------------- GMRES vectors
 
-constexpr int kReduceMaxBlocks = 1184;  // 8 per SM on 148 SMs
+// Per-column reductions: blocks of up to kReduceThreads threads (column x
+// point), kReduceUnroll points of each thread in flight, at most two blocks per
+// SM; the last block to finish adds the blocks' sums, in block order, with all
+// of its threads.  Bound by memory at large grids and by latency at small ones:
+// 2 x 512 threads x 4 points x 2 vectors x 16 bytes per SM cover HBM's latency,
+// and 296 block sums of up to 512 columns-per-thread slots are a handful of
+// loads per thread, where a second launch that added 1184 of them one after the
+// other took longer than the pass over the vectors.
+constexpr int kReduceMaxBlocks = 296;
+constexpr int kReduceThreads = 512;
+constexpr int kReduceUnroll = 4;
 
-__global__ void norms_partial_kernel(const z64* __restrict__ w, int64_t npoints, int k, double* partial) {
-    extern __shared__ double red[];
-    const int tx = threadIdx.x, ty = threadIdx.y;
-    double acc = 0;
-    for (int64_t p = blockIdx.x * (int64_t)blockDim.y + ty; p < npoints; p += (int64_t)gridDim.x * blockDim.y)
-        acc += cabs2(w[p * k + tx]);
-    red[ty * blockDim.x + tx] = acc;
+// Sum over this block's threads of a column; the result is in ty == 0.
+template <typename T>
+__device__ __forceinline__ T BlockColumnSum(T acc, T* red) {
+    const int at = threadIdx.y * blockDim.x + threadIdx.x;
+    red[at] = acc;
     __syncthreads();
     for (int s = blockDim.y / 2; s > 0; s >>= 1) {
-        if (ty < s) red[ty * blockDim.x + tx] += red[(ty + s) * blockDim.x + tx];
+        if (threadIdx.y < s) red[at] += red[at + s * blockDim.x];
         __syncthreads();
     }
-    if (ty == 0) partial[blockIdx.x * (int64_t)k + tx] = red[tx];
+    return red[threadIdx.x];
 }
 
-__global__ void sum_partial_real_kernel(const double* partial, int nblocks, int k, double* out, int sqrtOut) {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= k) return;
-    double acc = 0;
-    for (int b = 0; b < nblocks; ++b) acc += partial[(int64_t)b * k + r];
-    out[r] = sqrtOut ? sqrt(acc) : acc;
+__device__ __forceinline__ double LoadCg(const double* p) { return __ldcg(p); }
+__device__ __forceinline__ z64 LoadCg(const z64* p) {
+    const double2 v = __ldcg(reinterpret_cast<const double2*>(p));
+    return mk(v.x, v.y);
 }
 
-__global__ void mgs_step_kernel(z64* __restrict__ w, const z64* __restrict__ vprev, const z64* __restrict__ hprev,
-                                const z64* __restrict__ vnext, int64_t npoints, int k, z64* partial) {
+// acc of every thread of the grid -> out[column] (its square root on request).
+// `ticket` is zero before and after the launch.
+template <typename T, typename Finish>
+__device__ __forceinline__ void GridColumnSum(T acc, T* red, T* partial, int* ticket, const Finish& finish) {
+    __shared__ int last;
+    const int tx = threadIdx.x, ty = threadIdx.y, k = blockDim.x, nblocks = gridDim.x;
+    acc = BlockColumnSum(acc, red);
+    if (nblocks > 1) {
+        if (ty == 0) {
+            partial[blockIdx.x * (int64_t)k + tx] = acc;
+            __threadfence();
+        }
+        __syncthreads();
+        if (tx == 0 && ty == 0) {
+            const int before = atomicAdd(ticket, 1);
+            last = before == nblocks - 1;
+            if (last) *ticket = 0;
+            __threadfence();
+        }
+        __syncthreads();
+        if (!last) return;
+        acc = T();
+#pragma unroll 8
+        for (int b = ty; b < nblocks; b += blockDim.y) acc += LoadCg(partial + b * (int64_t)k + tx);
+        acc = BlockColumnSum(acc, red);
+    }
+    if (ty == 0) finish(tx, acc);
+}
+
+// w -= hprev vprev per column (when there is a vprev), then out = <vnext, w>
+// per column (kNorm false) or |w| (kNorm true).
+template <bool kUpdate, bool kNorm>
+__global__ void __launch_bounds__(1024) mgs_step_kernel(z64* __restrict__ w, const z64* __restrict__ vprev,
+                                                        const z64* __restrict__ hprev, const z64* __restrict__ vnext,
+                                                        int64_t npoints, int k, void* partial, int* ticket, void* out) {
     extern __shared__ z64 redc[];
     const int tx = threadIdx.x, ty = threadIdx.y;
-    const z64 h = vprev ? hprev[tx] : mk(0.0, 0.0);
+    const z64 h = kUpdate ? hprev[tx] : mk(0.0, 0.0);
     z64 acc = mk(0.0, 0.0);
-    for (int64_t p = blockIdx.x * (int64_t)blockDim.y + ty; p < npoints; p += (int64_t)gridDim.x * blockDim.y) {
-        const int64_t e = p * k + tx;
-        z64 wv = w[e];
-        if (vprev) {
-            wv -= h * vprev[e];
-            w[e] = wv;
+    const int64_t stride = (int64_t)gridDim.x * blockDim.y, step = stride * k;
+    int64_t p = blockIdx.x * (int64_t)blockDim.y + ty, e = p * k + tx;
+    auto point = [&](int64_t at, z64 wv, z64 vp, z64 vn) {
+        if (kUpdate) {
+            wv -= h * vp;
+            w[at] = wv;
         }
-        if (vnext) {
-            const z64 vv = vnext[e];
-            acc += mk(vv.re * wv.re + vv.im * wv.im, vv.re * wv.im - vv.im * wv.re);  // conj(v) w
+        if (kNorm) acc.re += cabs2(wv);
+        else acc += mk(vn.re * wv.re + vn.im * wv.im, vn.re * wv.im - vn.im * wv.re);  // conj(v) w
+    };
+    for (; p + (kReduceUnroll - 1) * stride < npoints; p += kReduceUnroll * stride, e += kReduceUnroll * step) {
+        z64 wv[kReduceUnroll], vp[kReduceUnroll], vn[kReduceUnroll];
+#pragma unroll
+        for (int i = 0; i < kReduceUnroll; ++i) {
+            wv[i] = w[e + i * step];
+            if (kUpdate) vp[i] = vprev[e + i * step];
+            if (!kNorm) vn[i] = vnext[e + i * step];
         }
+#pragma unroll
+        for (int i = 0; i < kReduceUnroll; ++i) point(e + i * step, wv[i], vp[i], vn[i]);
     }
-    if (!vnext) return;
-    redc[ty * blockDim.x + tx] = acc;
-    __syncthreads();
-    for (int s = blockDim.y / 2; s > 0; s >>= 1) {
-        if (ty < s) redc[ty * blockDim.x + tx] += redc[(ty + s) * blockDim.x + tx];
-        __syncthreads();
+    for (; p < npoints; p += stride, e += step)
+        point(e, w[e], kUpdate ? vprev[e] : acc, kNorm ? acc : vnext[e]);
+    if (kNorm) {
+        double* norm = static_cast<double*>(out);
+        GridColumnSum(acc.re, reinterpret_cast<double*>(redc), static_cast<double*>(partial), ticket,
+                      [&](int r, double v) { norm[r] = sqrt(v); });
+    } else {
+        z64* dot = static_cast<z64*>(out);
+        GridColumnSum(acc, redc, static_cast<z64*>(partial), ticket, [&](int r, z64 v) { dot[r] = v; });
     }
-    if (ty == 0) partial[blockIdx.x * (int64_t)k + tx] = redc[tx];
-}
-
-__global__ void sum_partial_complex_kernel(const z64* partial, int nblocks, int k, z64* out) {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= k) return;
-    z64 acc = mk(0.0, 0.0);
-    for (int b = 0; b < nblocks; ++b) acc += partial[(int64_t)b * k + r];
-    out[r] = acc;
 }
 
 __global__ void scale_columns_kernel(const z64* __restrict__ w, const double* __restrict__ s, z64* __restrict__ v,
@@ -409,17 +451,9 @@ __global__ void combine_kernel(const z64* __restrict__ x0, const z64* __restrict
     }
 }
 
-__global__ void axpy_columns_kernel(z64* __restrict__ w, const z64* __restrict__ v, const z64* __restrict__ h,
-                                    int64_t n, int k) {
-    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x) {
-        const int r = (int)(e % k);
-        w[e] -= h[r] * v[e];
-    }
-}
-
 inline dim3 ReduceBlockDim(int k) {
     int ty = 1;
-    while (ty * 2 * k <= 256) ty *= 2;
+    while (ty * 2 * k <= kReduceThreads) ty *= 2;
     return dim3(k, ty);
 }
 
@@ -515,27 +549,27 @@ int ReduceBlocks(int64_t npoints, int k) {
     return (int)std::max<int64_t>(1, std::min<int64_t>(CeilDiv(npoints, bd.y), kReduceMaxBlocks));
 }
 
-void LaunchNormsPartial(const z64* w, int64_t npoints, int k, double* partial, cudaStream_t st) {
+void LaunchNorms(const z64* w, int64_t npoints, int k, void* partial, int* ticket, double* out, cudaStream_t st) {
     const dim3 bd = ReduceBlockDim(k);
-    norms_partial_kernel<<<ReduceBlocks(npoints, k), bd, sizeof(double) * bd.x * bd.y, st>>>(w, npoints, k, partial);
+    mgs_step_kernel<false, true><<<ReduceBlocks(npoints, k), bd, sizeof(z64) * bd.x * bd.y, st>>>(
+        const_cast<z64*>(w), nullptr, nullptr, nullptr, npoints, k, partial, ticket, out);
     CUDA_LAUNCH_CHECK();
 }
 
-void LaunchSumPartialReal(const double* partial, int nblocks, int k, double* out, int sqrtOut, cudaStream_t st) {
-    sum_partial_real_kernel<<<CeilDiv(k, 64), 64, 0, st>>>(partial, nblocks, k, out, sqrtOut);
-    CUDA_LAUNCH_CHECK();
-}
-
-void LaunchMgsStep(z64* w, const z64* v_prev, const z64* h_prev, const z64* v_next, int64_t npoints, int k,
-                   z64* partial, cudaStream_t st) {
+void LaunchMgsStep(z64* w, const z64* vPrev, const z64* hPrev, const z64* vNext, int64_t npoints, int k, void* partial,
+                   int* ticket, z64* out, cudaStream_t st) {
     const dim3 bd = ReduceBlockDim(k);
-    mgs_step_kernel<<<ReduceBlocks(npoints, k), bd, sizeof(z64) * bd.x * bd.y, st>>>(w, v_prev, h_prev, v_next,
-                                                                                     npoints, k, partial);
+    const auto kernel = vPrev ? mgs_step_kernel<true, false> : mgs_step_kernel<false, false>;
+    kernel<<<ReduceBlocks(npoints, k), bd, sizeof(z64) * bd.x * bd.y, st>>>(w, vPrev, hPrev, vNext, npoints, k, partial,
+                                                                          ticket, out);
     CUDA_LAUNCH_CHECK();
 }
 
-void LaunchSumPartialComplex(const z64* partial, int nblocks, int k, z64* out, cudaStream_t st) {
-    sum_partial_complex_kernel<<<CeilDiv(k, 64), 64, 0, st>>>(partial, nblocks, k, out);
+void LaunchMgsNorm(z64* w, const z64* vPrev, const z64* hPrev, int64_t npoints, int k, void* partial, int* ticket,
+                   double* out, cudaStream_t st) {
+    const dim3 bd = ReduceBlockDim(k);
+    mgs_step_kernel<true, true><<<ReduceBlocks(npoints, k), bd, sizeof(z64) * bd.x * bd.y, st>>>(
+        w, vPrev, hPrev, nullptr, npoints, k, partial, ticket, out);
     CUDA_LAUNCH_CHECK();
 }
 
@@ -549,12 +583,6 @@ void LaunchCombine(const z64* x0, const z64* V, int64_t vstride, const z64* y, i
                    int k, cudaStream_t st) {
     const int64_t n = npoints * k;
     combine_kernel<<<ElementwiseGrid(n), kThreads, 0, st>>>(x0, V, vstride, y, j1, x, n, k);
-    CUDA_LAUNCH_CHECK();
-}
-
-void LaunchAxpyColumns(z64* w, const z64* v, const z64* h, int64_t npoints, int k, cudaStream_t st) {
-    const int64_t n = npoints * k;
-    axpy_columns_kernel<<<ElementwiseGrid(n), kThreads, 0, st>>>(w, v, h, n, k);
     CUDA_LAUNCH_CHECK();
 }
 

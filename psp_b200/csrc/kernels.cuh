@@ -243,21 +243,22 @@ void LaunchFlowTc(const FlowFront<float>* fr, const FlowTile* tiles, int n, int 
 
 // ------------------------------------------------------------------ GMRES vectors
 
-// Per-RHS reductions over natural-order [N][k] vectors; partial sums per block
-// land in `partial` (gridDim x k) and a second pass sums them in fixed order.
+// Per-RHS reductions over natural-order [N][k] vectors, one launch each: the
+// blocks' sums land in `partial` (gridDim x k) and the last block to finish adds
+// them in block order (`ticket`: zero before, and again after, every launch).
 int ReduceBlocks(int64_t npoints, int k);
-void LaunchNormsPartial(const z64* w, int64_t npoints, int k, double* partial, cudaStream_t st);
-void LaunchSumPartialReal(const double* partial, int nblocks, int k, double* out, int sqrtOut, cudaStream_t st);
-// w -= h_prev (.) v_prev (if v_prev) and partial dots conj(v_next) . w
-void LaunchMgsStep(z64* w, const z64* v_prev, const z64* h_prev, const z64* v_next, int64_t npoints, int k,
-                   z64* partial, cudaStream_t st);
-void LaunchSumPartialComplex(const z64* partial, int nblocks, int k, z64* out, cudaStream_t st);
+// out[r] := |w[:, r]|
+void LaunchNorms(const z64* w, int64_t npoints, int k, void* partial, int* ticket, double* out, cudaStream_t st);
+// w -= hPrev (.) vPrev (if vPrev), out[r] := conj(vNext[:, r]) . w[:, r]
+void LaunchMgsStep(z64* w, const z64* vPrev, const z64* hPrev, const z64* vNext, int64_t npoints, int k, void* partial,
+                   int* ticket, z64* out, cudaStream_t st);
+// w -= hPrev (.) vPrev, out[r] := |w[:, r]|
+void LaunchMgsNorm(z64* w, const z64* vPrev, const z64* hPrev, int64_t npoints, int k, void* partial, int* ticket,
+                   double* out, cudaStream_t st);
 // v := w / s (per RHS, s real)
 void LaunchScaleColumns(const z64* w, const double* s, z64* v, int64_t npoints, int k, cudaStream_t st);
 // x := x0 + sum_i y[i,r] V_i[:,r]
 void LaunchCombine(const z64* x0, const z64* V, int64_t vstride, const z64* y, int j1, z64* x, int64_t npoints,
                    int k, cudaStream_t st);
-// w := w - h (.) v   (final MGS axpy)
-void LaunchAxpyColumns(z64* w, const z64* v, const z64* h, int64_t npoints, int k, cudaStream_t st);
 
 }  // namespace psp_b200

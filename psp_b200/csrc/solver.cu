@@ -1454,7 +1454,8 @@ void Helmholtz::EnsureWorkspace(int k, int m, bool withCols) {
     const size_t partial = al((size_t)ReduceBlocks(NumUnknowns(), k) * k * sizeof(z64));
     const size_t scal = al((size_t)(2 * k) * sizeof(double) + (size_t)(m + 1) * k * sizeof(z64));
     const size_t ybytes = al((size_t)m * k * sizeof(z64));
-    const size_t total = vec * (4 + m + (withCols ? 1 : 0)) + partial + scal + ybytes;
+    const size_t ticket = al(sizeof(int));
+    const size_t total = vec * (4 + m + (withCols ? 1 : 0)) + partial + ticket + scal + ybytes;
     unsigned char* p = static_cast<unsigned char*>(Scratch(total));
     auto take = [&](size_t b) { unsigned char* q = p; p += b; return q; };
     wsCols_ = withCols ? reinterpret_cast<z64*>(take(vec)) : nullptr;
@@ -1464,6 +1465,7 @@ void Helmholtz::EnsureWorkspace(int k, int m, bool withCols) {
     wsB_ = reinterpret_cast<z64*>(take(vec));
     wsV_ = reinterpret_cast<z64*>(take(vec * m));
     wsPartial_ = take(partial);
+    wsTicket_ = take(ticket);
     wsScal_ = take(scal);
     wsY_ = reinterpret_cast<z64*>(take(ybytes));
 }
@@ -1625,19 +1627,15 @@ void Helmholtz::SolveBlock(z64* B, int k, int m, double relTol, SolveStats* stat
     double* dDelta = dNorm + k;
     z64* dH = reinterpret_cast<z64*>(dDelta + k);
     z64* dY = wsY_;
-    double* partialR = static_cast<double*>(wsPartial_);
-    z64* partialC = static_cast<z64*>(wsPartial_);
-    const int nblk = ReduceBlocks(N, k);
+    int* ticket = static_cast<int*>(wsTicket_);
+    CUDA_CHECK(cudaMemsetAsync(ticket, 0, sizeof(int), st));
     const double* vel = dVel_.as<double>();
     // per-kernel profiling (when on) of the GMRES vector kernels: algorithmic
     // bytes = the [N][k] vectors each launch reads and writes
     const double vb = 16.0 * (double)nk;
     auto norms = [&](const z64* v, double* out) {
-        {
-            ProfScope ps(st, kProfVector, 4.0 * nk, vb);
-            LaunchNormsPartial(v, N, k, partialR, st);
-        }
-        LaunchSumPartialReal(partialR, nblk, k, out, 1, st);
+        ProfScope ps(st, kProfVector, 4.0 * nk, vb);
+        LaunchNorms(v, N, k, wsPartial_, ticket, out, st);
     };
     auto fetch = [&](void* dst, const void* src, size_t bytes) {
         CUDA_CHECK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st));
@@ -1725,18 +1723,15 @@ void Helmholtz::SolveBlock(z64* B, int k, int m, double relTol, SolveStats* stat
             precond();
             phases.Begin(st);
             for (int i = 0; i <= j; ++i) {
-                {
-                    ProfScope ps(st, kProfVector, (i > 0 ? 16.0 : 8.0) * nk, (i > 0 ? 4 : 2) * vb);
-                    LaunchMgsStep(w, i > 0 ? V + (size_t)(i - 1) * nk : nullptr,
-                                  i > 0 ? dH + (size_t)(i - 1) * k : nullptr, V + (size_t)i * nk, N, k, partialC, st);
-                }
-                LaunchSumPartialComplex(partialC, nblk, k, dH + (size_t)i * k, st);
+                ProfScope ps(st, kProfVector, (i > 0 ? 16.0 : 8.0) * nk, (i > 0 ? 4 : 2) * vb);
+                LaunchMgsStep(w, i > 0 ? V + (size_t)(i - 1) * nk : nullptr,
+                              i > 0 ? dH + (size_t)(i - 1) * k : nullptr, V + (size_t)i * nk, N, k, wsPartial_, ticket,
+                              dH + (size_t)i * k, st);
             }
             {
-                ProfScope ps(st, kProfVector, 8.0 * nk, 3 * vb);
-                LaunchAxpyColumns(w, V + (size_t)j * nk, dH + (size_t)j * k, N, k, st);
+                ProfScope ps(st, kProfVector, 12.0 * nk, 3 * vb);
+                LaunchMgsNorm(w, V + (size_t)j * nk, dH + (size_t)j * k, N, k, wsPartial_, ticket, dDelta, st);
             }
-            norms(w, dDelta);
             phases.End(st, kProfVector, 8.0 * 2 * (j + 1) * nk, 16.0 * (3 * (j + 1) + 2) * nk);
             hcol.resize((size_t)(j + 1) * k);
             fetch(hcol.data(), dH, (size_t)(j + 1) * k * sizeof(z64));

@@ -210,6 +210,7 @@ private:
     z64 *wsX_ = nullptr, *wsX0_ = nullptr, *wsW_ = nullptr, *wsB_ = nullptr, *wsV_ = nullptr;
     z64 *wsCols_ = nullptr, *wsY_ = nullptr;
     void* wsPartial_ = nullptr;
+    void* wsTicket_ = nullptr;
     void* wsScal_ = nullptr;
 };
 
