@@ -153,6 +153,7 @@ void LaunchLdlTrsm(const FactorFront<R>* fronts, const int2* tasks, int n, int J
 
 struct PanelIO {
     const int* ndToNat;
+    const int* natToNd;
     int nxy, nx, nz;
     int ldk;         // row stride (complex entries per point) of the natural-order grid
     int padding;     // leading planes of the subproblem that are artificial padding
@@ -230,7 +231,7 @@ void PrepareFlowKernels();
 template <typename R>
 void EncodeFlowMaps(const cpx<R>* G, int s, int u, int ldg, void* out);
 template <typename R>
-void LaunchFlowGather(const z64* B, cpx<R>* rnd, int nSub, int k, const PanelIO& io, cudaStream_t st);
+void LaunchFlowGather(const z64* B, cpx<R>* rnd, int own, int k, const PanelIO& io, cudaStream_t st);
 template <typename R>
 void LaunchFlow(const FlowFront<R>* fr, const FlowTile* tiles, int n, int k, z64* B, const PanelIO& io,
                 const FlowWork& w, cudaStream_t st);

@@ -269,6 +269,7 @@ private:
         int cols = 0;     // right-hand sides per tile
         DeviceBuffer rnd, W, X, planes, partials, counters, done;
         int planesClass = -1;  // class whose unwritten plane rows are zero
+        int rndPanel = -1;     // last panel gathered: its unwritten (padding) rows of rnd are zero
         TaskArena arena;
         // per class the ordered tile list (arena offset) and its work, per
         // panel its fronts
@@ -839,7 +840,7 @@ typename FactorStore<R>::SolvePlan& FactorStore<R>::Plan(int k) {
     P.W.Allocate((size_t)maxSub * k * sizeof(cpx<R>));
     P.X.Allocate((size_t)maxSub * k * sizeof(cpx<R>));
     P.planes.Allocate((size_t)maxRows * k * sizeof(cpx<R>));
-    P.planesClass = -1;
+    P.planesClass = P.rndPanel = -1;
     P.arena.host.clear();
     P.panelFronts.assign(np, 0);
     P.mapsHost.assign((size_t)np * nn_, {});
@@ -1024,6 +1025,7 @@ void FactorStore<R>::SolvePanel(z64* B, int ldk, int k, int p, int inMode, int o
     cudaStream_t st = h_.stream_;
     PanelIO io;
     io.ndToNat = h_.dNdToNat_[c].as<int>();
+    io.natToNd = h_.dNatToNd_[c].as<int>();
     io.nx = an_.disc.nx;
     io.nxy = an_.disc.nx * an_.disc.ny;
     io.nz = an_.disc.nz - zBase;  // kernels index plane nz - 1 - v: relative to the slab's first plane
@@ -1051,7 +1053,11 @@ void FactorStore<R>::SolvePanel(z64* B, int ldk, int k, int p, int inMode, int o
             CUDA_CHECK(cudaMemsetAsync(P.planes.p, 0, P.planes.bytes, st));
             P.planesClass = c;
         }
-        LaunchFlowGather<R>(B, P.rnd.template as<cpx<R>>(), an_.cls[c].nSub, k, io, st);
+        // (the bottom panel shares its class with the inner ones, but has no padding)
+        if (io.padding > 0 && (P.rndPanel < 0 || g.Class(P.rndPanel) != c || g.Padding(P.rndPanel) != io.padding))
+            CUDA_CHECK(cudaMemsetAsync(P.rnd.p, 0, P.rnd.bytes, st));
+        P.rndPanel = p;
+        LaunchFlowGather<R>(B, P.rnd.template as<cpx<R>>(), an_.cls[c].nSub - io.padding * io.nxy, k, io, st);
     }
     ProfScope ps(st, kProfSolveGemm, P.flops[c], P.bytes[c]);
     const FlowFront<R>* fr = P.arena.template At<FlowFront<R>>(P.panelFronts[p]);
@@ -1088,6 +1094,7 @@ void FactorStore<R>::Sweep(z64* B, int ldk, int k, bool useGraph) {
         if (g.B == B && g.ldk == ldk && g.k == k) {
             CUDA_CHECK(cudaGraphLaunch(g.exec, h_.stream_));
             P.planesClass = an_.geom.Class(0);  // of the sweep's last panel solve
+            P.rndPanel = 0;
             return;
         }
     if (graphs_.size() >= 8) {  // graphs of earlier work vectors (the scratch moved)
@@ -1096,7 +1103,7 @@ void FactorStore<R>::Sweep(z64* B, int ldk, int k, bool useGraph) {
     }
     cudaGraph_t graph;
     CUDA_CHECK(cudaStreamBeginCapture(h_.stream_, cudaStreamCaptureModeThreadLocal));
-    P.planesClass = -1;  // the graph clears the planes whatever ran before it
+    P.planesClass = P.rndPanel = -1;  // the graph clears the planes whatever ran before it
     SweepEager(B, ldk, k);
     CUDA_CHECK(cudaStreamEndCapture(h_.stream_, &graph));
     SweepGraph g{B, ldk, k, nullptr};
@@ -1245,6 +1252,7 @@ void Helmholtz::BuildTables() {
         if (!an_.classUsed[c]) continue;
         const ClassStructure& cs = an_.cls[c];
         UploadVector(dNdToNat_[c], cs.ndToNat, stream_);
+        UploadVector(dNatToNd_[c], cs.natToNd, stream_);
         UploadVector(dNbrRows_[c], cs.nbrRows, stream_);
         UploadVector(dRel_[c], cs.rel, stream_);
         UploadVector(dLower_[c], cs.lower, stream_);

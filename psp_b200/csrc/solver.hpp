@@ -170,7 +170,7 @@ public:
     AssemblyParams ap_{};
     DeviceBuffer dS1_, dS2_, dS3_, dS3a_;   // values and reciprocals back to back
     DeviceBuffer dVel_;
-    DeviceBuffer dNdToNat_[3], dNbrRows_[3], dRel_[3], dLower_[3];
+    DeviceBuffer dNdToNat_[3], dNatToNd_[3], dNbrRows_[3], dRel_[3], dLower_[3];
     std::vector<int> s3aOff_;                // per panel
     Analysis an_;
     double damping_;

@@ -652,32 +652,6 @@ __device__ void ComputeRole(int k, unsigned char* smem, Sync<R>& S, z64* B, cons
 
 // ------------------------------------------------------------------ kernels
 
-// Entry (col, r) of a panel's right-hand side: row `col` of the subproblem's
-// ordering, with the sweep's coupling to the neighbouring panel.
-template <typename R>
-__device__ __forceinline__ cpx<R> PanelRhs(const PanelIO& io, const z64* __restrict__ B, int col, int r) {
-    const int pn = io.ndToNat[col];
-    const int xy = pn % io.nxy, vl = pn / io.nxy;
-    if (vl < io.padding) return mk<R>(0, 0);
-    const int v = io.vOffset + vl;
-    const int64_t nat = xy + (int64_t)(io.nz - 1 - v) * io.nxy;
-    const int x = xy % io.nx, y = xy / io.nx;
-    const StencilParams& sp = io.sp;
-    if (io.inMode == 2) {
-        if (v != io.highV) return mk<R>(0, 0);
-        const z64 cz = sp.s1[x + 1] * sp.s2[y + 1];
-        const z64 coef = sp.ihz2 * (cz * (sp.is3[v + 2] + sp.is3[v + 1]));
-        return ccast<R>(coef * B[(nat - io.nxy) * io.ldk + r]);
-    }
-    z64 val = B[nat * io.ldk + r];
-    if (io.inMode == 1 && v == io.lowV) {
-        const z64 cz = sp.s1[x + 1] * sp.s2[y + 1];
-        const z64 coef = sp.ihz2 * (cz * (sp.is3[v] + sp.is3[v + 1]));
-        val += coef * B[(nat + io.nxy) * io.ldk + r];
-    }
-    return ccast<R>(val);
-}
-
 template <typename R, int NC>
 __global__ void __launch_bounds__(kThreads, 2) sweep_flow_kernel(const FlowFront<R>* __restrict__ fr,
                                                                  const FlowTile* __restrict__ tiles, int n, int k,
@@ -714,16 +688,54 @@ __global__ void __launch_bounds__(kThreads, 2) sweep_flow_kernel(const FlowFront
 
 // The panel's right-hand sides in the subproblem's nested-dissection order,
 // rounded to the factors' precision: the planes' own entries with the sweep's
-// panel coupling folded in, zero on the artificial padding.
-template <typename R>
-__global__ void __launch_bounds__(256) flow_gather_kernel(const z64* __restrict__ B, cpx<R>* __restrict__ rnd, int nSub,
-                                                          int k, const __grid_constant__ PanelIO io) {
+// panel coupling folded in.  The rows of the artificial padding are zero and
+// stay zero; they are not written.
+//
+// Bound by memory: points in natural order, so that the grid is read in long
+// runs (16 k bytes per point) and rows of 8 k or 16 k bytes are scattered; a
+// thread keeps its columns (kVec of them, 16 bytes of the result in complex
+// single), two points in flight.  With rows in the subproblem's order, padding
+// included, and a 64-bit division per entry it took 26 us at 96 x 96, k = 32, and
+// 20 us at 116 x 116, k = 16 (mean over a sweep's panel solves); now 16 and 13 us.
+template <typename R, int kVec>
+__global__ void __launch_bounds__(256) flow_gather_kernel(const z64* __restrict__ B, cpx<R>* __restrict__ rnd, int own,
+                                                          int k, int units, const __grid_constant__ PanelIO io) {
     PdlWait();
     PdlTrigger();  // after the wait: the tree kernel may copy factors as soon as it starts
-    const int64_t total = (int64_t)nSub * k;
-    for (int64_t e = blockIdx.x * 256 + threadIdx.x; e < total; e += (int64_t)gridDim.x * 256) {
-        const int i = (int)(e / k), r = (int)(e - (int64_t)i * k);
-        rnd[e] = PanelRhs<R>(io, B, i, r);
+    const StencilParams& sp = io.sp;
+    const int rows = 256 / units, row = threadIdx.x / units, r = (blockIdx.y * units + threadIdx.x % units) * kVec;
+    if (row >= rows || r >= k) return;
+#pragma unroll 2
+    for (int i = blockIdx.x * rows + row; i < own; i += gridDim.x * rows) {
+        const int first = io.padding * io.nxy, plane = i / io.nxy, xy = i - plane * io.nxy;
+        const int at = __ldg(io.natToNd + first + i);
+        const int v = io.vOffset + io.padding + plane;
+        const z64* b = B + (xy + (int64_t)(io.nz - 1 - v) * io.nxy) * io.ldk + r;
+        const int64_t up = (int64_t)io.nxy * io.ldk;  // the plane before in v
+        z64 val[kVec];
+        if (io.inMode != 2) {
+#pragma unroll
+            for (int c = 0; c < kVec; ++c) val[c] = b[c];
+            if (io.inMode == 1 && v == io.lowV) {
+                const z64 coef = sp.ihz2 * (sp.s1[xy % io.nx + 1] * sp.s2[xy / io.nx + 1] * (sp.is3[v] + sp.is3[v + 1]));
+#pragma unroll
+                for (int c = 0; c < kVec; ++c) val[c] += coef * b[up + c];
+            }
+        } else if (v == io.highV) {
+            const z64 coef = sp.ihz2 * (sp.s1[xy % io.nx + 1] * sp.s2[xy / io.nx + 1] * (sp.is3[v + 2] + sp.is3[v + 1]));
+#pragma unroll
+            for (int c = 0; c < kVec; ++c) val[c] = coef * b[c - up];
+        } else {
+#pragma unroll
+            for (int c = 0; c < kVec; ++c) val[c] = mk(0.0, 0.0);
+        }
+        cpx<R>* const dst = rnd + (int64_t)at * k + r;
+        if constexpr (kVec == 2) {
+            const c32 a = ccast<float>(val[0]), c = ccast<float>(val[1]);
+            *reinterpret_cast<float4*>(dst) = make_float4(a.re, a.im, c.re, c.im);
+        } else {
+            *dst = ccast<R>(val[0]);
+        }
     }
 }
 
@@ -798,10 +810,12 @@ void EncodeFlowMaps(const cpx<R>* G, int s, int u, int ldg, void* out) {
 }
 
 template <typename R>
-void LaunchFlowGather(const z64* B, cpx<R>* rnd, int nSub, int k, const PanelIO& io, cudaStream_t st) {
-    const int64_t total = (int64_t)nSub * k;
-    const unsigned grid = std::min<unsigned>(CeilDiv(total, 256), 8 * g_flowSMs);
-    LaunchPdl(flow_gather_kernel<R>, dim3(grid), dim3(256), 0, st, B, rnd, nSub, k, io);
+void LaunchFlowGather(const z64* B, cpx<R>* rnd, int own, int k, const PanelIO& io, cudaStream_t st) {
+    // two columns of complex single are 16 bytes when rows are
+    const int vec = sizeof(R) == 4 && k % 2 == 0 ? 2 : 1, units = std::min(k / vec, 256);
+    const dim3 grid(std::min<unsigned>(CeilDiv(own, 256 / units), 16 * g_flowSMs), CeilDiv(k / vec, units));
+    if (vec == 2) LaunchPdl(flow_gather_kernel<R, sizeof(R) == 4 ? 2 : 1>, grid, dim3(256), 0, st, B, rnd, own, k, units, io);
+    else LaunchPdl(flow_gather_kernel<R, 1>, grid, dim3(256), 0, st, B, rnd, own, k, units, io);
 }
 
 template <typename R>
