@@ -11,6 +11,12 @@ namespace {
 
 constexpr int kThreads = 256;
 
+__device__ __forceinline__ double LoadCg(const double* p) { return __ldcg(p); }
+__device__ __forceinline__ z64 LoadCg(const z64* p) {
+    const double2 v = __ldcg(reinterpret_cast<const double2*>(p));
+    return mk(v.x, v.y);
+}
+
 // Face and centre terms of one stencil row (initialize_finalize.hpp:527-587
 // and 589-651).  s3M and the three s3 reciprocals come from either the global
 // or the panel's artificial table; omega is omega (+ i*damping for panels).
@@ -36,14 +42,23 @@ __device__ __forceinline__ Terms StencilAt(const StencilParams& sp, int x, int y
 
 // ---------------------------------------------------------------- stencil apply
 
-constexpr int kApplyTX = 64;
+// A block applies the operator to kApplyTX points of a row: one thread per
+// point for the coefficients (products and quotients of the stretch tables),
+// then one per column and point, all seven entries in flight.  Eight blocks per
+// SM hide the first part behind the second.  Bound by memory: 140 x 140 x 80,
+// k = 32 (0.8 GB in, 0.8 GB out, b in every second launch): 0.45 ms with 64
+// points on 256 threads, most of them idle through the coefficients, now 0.42 ms
+// (4.8 TB/s); two or four planes per block with the column in registers have
+// fewer warps in flight and take 0.44 and 0.69 ms.
+constexpr int kApplyTX = 128;
 
-__global__ void __launch_bounds__(kThreads) helmholtz_apply_kernel(const z64* __restrict__ x, z64* __restrict__ y,
-                                                                   const z64* __restrict__ b,
-                                                                   const double* __restrict__ vel, StencilParams sp,
-                                                                   int k, int zFirst, int zSlab) {
+// out(e, (A x) at entry e of the row piece); `base` is the piece's first point
+// in x's storage, `ready` runs before the first use of x.
+template <typename Ready, typename Out>
+__device__ __forceinline__ void ApplyRow(const z64* __restrict__ x, const double* __restrict__ vel,
+                                         const StencilParams& sp, int k, int x0, int yy, int zz, int64_t base,
+                                         const Ready& ready, const Out& out) {
     __shared__ z64 coef[kApplyTX][7];
-    const int x0 = blockIdx.x * kApplyTX, yy = blockIdx.y, zz = zFirst + (int)blockIdx.z;
     const int nx = sp.nx, ny = sp.ny, nz = sp.nz;
     const int64_t nxy = (int64_t)nx * ny;
     const int npts = min(kApplyTX, nx - x0);
@@ -52,30 +67,83 @@ __global__ void __launch_bounds__(kThreads) helmholtz_apply_kernel(const z64* __
         const int xx = x0 + threadIdx.x;
         const Terms t = StencilAt(sp, xx, yy, sp.s3[v + 1], sp.is3[v], sp.is3[v + 1], sp.is3[v + 2],
                                   mk(sp.omega, 0.0), vel[xx + yy * (int64_t)nx + zz * nxy]);
-        coef[threadIdx.x][0] = t.c;
-        coef[threadIdx.x][1] = -t.xL;
-        coef[threadIdx.x][2] = -t.xR;
-        coef[threadIdx.x][3] = -t.yL;
-        coef[threadIdx.x][4] = -t.yR;
-        coef[threadIdx.x][5] = -t.vL;
-        coef[threadIdx.x][6] = -t.vR;
+        z64* c = coef[threadIdx.x];
+        c[0] = t.c;
+        c[1] = -t.xL;
+        c[2] = -t.xR;
+        c[3] = -t.yL;
+        c[4] = -t.yR;
+        c[5] = -t.vL;
+        c[6] = -t.vR;
     }
+    ready();
     __syncthreads();
-    const int64_t base = x0 + yy * (int64_t)nx + (zz - zSlab) * nxy;  // storage: planes from zSlab
     const int64_t sx = k, sy = (int64_t)nx * k, sz = nxy * k;
-    for (int e = threadIdx.x; e < npts * k; e += blockDim.x) {
-        const int p = e / k, r = e - p * k;
-        const int xx = x0 + p;
-        const int64_t idx = (base + p) * k + r;
-        const z64* xp = x + idx;
-        z64 acc = coef[p][0] * xp[0];
-        if (xx > 0) cfma(acc, coef[p][1], xp[-sx]);
-        if (xx + 1 < nx) cfma(acc, coef[p][2], xp[sx]);
-        if (yy > 0) cfma(acc, coef[p][3], xp[-sy]);
-        if (yy + 1 < ny) cfma(acc, coef[p][4], xp[sy]);
-        if (zz + 1 < nz) cfma(acc, coef[p][5], xp[sz]);   // v-1 neighbour
-        if (zz > 0) cfma(acc, coef[p][6], xp[-sz]);       // v+1 neighbour
-        y[idx] = b ? b[idx] - acc : acc;
+    const z64* const row = x + base * k;
+    for (int e = threadIdx.x; e < npts * k; e += kApplyTX) {
+        const int p = e / k, xx = x0 + p;
+        const z64 none = mk(0.0, 0.0);
+        const z64* q = row + e;
+        const z64 c = q[0];
+        const z64 xl = xx > 0 ? q[-sx] : none, xr = xx + 1 < nx ? q[sx] : none;
+        const z64 yl = yy > 0 ? q[-sy] : none, yr = yy + 1 < ny ? q[sy] : none;
+        const z64 zr = zz + 1 < nz ? q[sz] : none, zl = zz > 0 ? q[-sz] : none;
+        const z64* f = coef[p];
+        z64 acc = f[0] * c;
+        if (xx > 0) cfma(acc, f[1], xl);
+        if (xx + 1 < nx) cfma(acc, f[2], xr);
+        if (yy > 0) cfma(acc, f[3], yl);
+        if (yy + 1 < ny) cfma(acc, f[4], yr);
+        if (zz + 1 < nz) cfma(acc, f[5], zr);  // v-1 neighbour
+        if (zz > 0) cfma(acc, f[6], zl);       // v+1 neighbour
+        out(e, acc);
+    }
+}
+
+// Planes zFirst ..; storage from plane zSlab.
+__global__ void __launch_bounds__(kApplyTX, 8) helmholtz_apply_kernel(const z64* __restrict__ x, z64* __restrict__ y,
+                                                                      const z64* __restrict__ b,
+                                                                      const double* __restrict__ vel, StencilParams sp,
+                                                                      int k, int zFirst, int zSlab) {
+    const int x0 = blockIdx.x * kApplyTX, yy = blockIdx.y, zz = zFirst + (int)blockIdx.z;
+    const int64_t base = x0 + yy * (int64_t)sp.nx + (zz - zSlab) * ((int64_t)sp.nx * sp.ny);
+    ApplyRow(x, vel, sp, k, x0, yy, zz, base, [] {}, [&](int e, z64 v) {
+        const int64_t idx = base * k + e;
+        y[idx] = b ? b[idx] - v : v;
+    });
+}
+
+// One step of B := A B: planes zApply .. of A B go to `ring` (plane z in slot
+// z mod ringPlanes), planes zCopy .. of it, of an earlier step, to B.  The
+// stencil reads one plane beyond its slab on either side, which no step before
+// the next has overwritten.  Bound by memory: 4 x 16 bytes per entry.
+__global__ void __launch_bounds__(kApplyTX, 8) helmholtz_in_place_kernel(z64* __restrict__ B, z64* __restrict__ ring,
+                                                                         const double* __restrict__ vel,
+                                                                         StencilParams sp, int k, int zApply,
+                                                                         int numApply, int zCopy, int ringPlanes) {
+    const int x0 = blockIdx.x * kApplyTX, yy = blockIdx.y;
+    const bool apply = (int)blockIdx.z < numApply;
+    const int zz = apply ? zApply + (int)blockIdx.z : zCopy + (int)blockIdx.z - numApply;
+    const int64_t nxy = (int64_t)sp.nx * sp.ny, row = x0 + yy * (int64_t)sp.nx, base = row + zz * nxy;
+    z64* const slot = ring + (row + zz % ringPlanes * nxy) * k;
+    auto ready = [] {
+        PdlWait();
+        PdlTrigger();
+    };
+    if (apply) {
+        ApplyRow(B, vel, sp, k, x0, yy, zz, base, ready, [&](int e, z64 v) { slot[e] = v; });
+    } else {
+        ready();
+        const int n = min(kApplyTX, sp.nx - x0) * k;
+        for (int e = threadIdx.x; e < n; e += 4 * kApplyTX) {
+            z64 v[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (e + i * kApplyTX < n) v[i] = LoadCg(slot + e + i * kApplyTX);
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (e + i * kApplyTX < n) B[base * k + e + i * kApplyTX] = v[i];
+        }
     }
 }
 
@@ -354,12 +422,6 @@ __device__ __forceinline__ T BlockColumnSum(T acc, T* red) {
     return red[threadIdx.x];
 }
 
-__device__ __forceinline__ double LoadCg(const double* p) { return __ldcg(p); }
-__device__ __forceinline__ z64 LoadCg(const z64* p) {
-    const double2 v = __ldcg(reinterpret_cast<const double2*>(p));
-    return mk(v.x, v.y);
-}
-
 // acc of every thread of the grid -> out[column] (its square root on request).
 // `ticket` is zero before and after the launch.
 template <typename T, typename Finish>
@@ -472,16 +534,43 @@ void LaunchGemmCfg(const GemmOp<R>* ops, const GemmTile* tiles, int numTiles, cu
 
 void LaunchHelmholtzApply(const z64* x, z64* y, const z64* b, const double* vel, const StencilParams& sp, int k,
                           cudaStream_t st) {
-    dim3 grid(CeilDiv(sp.nx, kApplyTX), sp.ny, sp.nz);
-    helmholtz_apply_kernel<<<grid, kThreads, 0, st>>>(x, y, b, vel, sp, k, 0, 0);
-    CUDA_LAUNCH_CHECK();
+    LaunchHelmholtzApplyPlanes(x, y, b, vel, sp, k, 0, sp.nz, 0, st);
 }
 
 void LaunchHelmholtzApplyPlanes(const z64* x, z64* y, const z64* b, const double* vel, const StencilParams& sp,
                                 int k, int zFirst, int zCount, int zSlab, cudaStream_t st) {
     dim3 grid(CeilDiv(sp.nx, kApplyTX), sp.ny, zCount);
-    helmholtz_apply_kernel<<<grid, kThreads, 0, st>>>(x, y, b, vel, sp, k, zFirst, zSlab);
+    helmholtz_apply_kernel<<<grid, kApplyTX, 0, st>>>(x, y, b, vel, sp, k, zFirst, zSlab);
     CUDA_LAUNCH_CHECK();
+}
+
+// Planes of one step of the in-place apply.  Up to kInPlaceRing bytes (0.6 % of
+// the device's memory) A B is one step and its copy: 400 MB take 320 us, against
+// 426, 414 us in slabs of 32, 64 MB, whose launches cost more than their shorter
+// way through L2 saves.  Larger grids go in slabs of a third of that.
+constexpr size_t kInPlaceRing = size_t(1) << 30;
+int InPlaceSlabPlanes(const StencilParams& sp, int k) {
+    const size_t plane = (size_t)sp.nx * sp.ny * k * sizeof(z64);
+    return plane * sp.nz <= kInPlaceRing ? sp.nz : (int)std::max<size_t>(1, kInPlaceRing / 3 / plane);
+}
+
+size_t InPlaceApplyBytes(const StencilParams& sp, int k) {
+    const size_t plane = (size_t)sp.nx * sp.ny * k * sizeof(z64);
+    return plane * std::min(sp.nz, 3 * InPlaceSlabPlanes(sp, k));
+}
+
+void LaunchHelmholtzInPlace(z64* B, void* ring, const double* vel, const StencilParams& sp, int k, cudaStream_t st) {
+    const int planes = InPlaceSlabPlanes(sp, k), slabs = (int)CeilDiv(sp.nz, planes);
+    const int ringPlanes = std::min(sp.nz, 3 * planes);
+    const int behind = slabs > 1 ? 2 : 1;
+    auto count = [&](int s) { return s < 0 || s >= slabs ? 0 : std::min(planes, sp.nz - s * planes); };
+    for (int s = 0; s < slabs + behind; ++s) {
+        const int na = count(s), nc = count(s - behind);
+        if (na + nc == 0) continue;
+        LaunchPdl(helmholtz_in_place_kernel, dim3(CeilDiv(sp.nx, kApplyTX), sp.ny, na + nc), dim3(kApplyTX), 0, st, B,
+                  static_cast<z64*>(ring), vel, sp, k, s * planes, na, (s - behind) * planes, ringPlanes);
+        CUDA_LAUNCH_CHECK();
+    }
 }
 
 void LaunchVelocityGradient(const z64* U, const z64* Z, const double* vel, const StencilParams& sp, int k,

@@ -32,6 +32,10 @@ void LaunchHelmholtzApply(const z64* x, z64* y, const z64* b, const double* vel,
 void LaunchHelmholtzApplyPlanes(const z64* x, z64* y, const z64* b, const double* vel, const StencilParams& sp,
                                 int k, int zFirst, int zCount, int zSlab, cudaStream_t st);
 
+// B := A B by slabs of planes; `ring` holds InPlaceApplyBytes.
+size_t InPlaceApplyBytes(const StencilParams& sp, int k);
+void LaunchHelmholtzInPlace(z64* B, void* ring, const double* vel, const StencilParams& sp, int k, cudaStream_t st);
+
 // grad[i] (+)= -Re( dA_ii/dvel_i * sum_r Z[i,r] U[i,r] ) for natural-order
 // [N][k] grids: the velocity gradient of a real misfit whose forward fields
 // are U and whose adjoint fields (A Z = conj of the misfit's field gradient)

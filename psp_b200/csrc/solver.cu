@@ -1302,7 +1302,14 @@ void Helmholtz::Finalize() {
     f64_.reset();
     f32_.reset();
     pool_.Release();
+    ReleaseApplyRing();
     initialized_ = false;
+}
+
+void Helmholtz::ReleaseApplyRing() {
+    std::lock_guard<std::mutex> lock(applyMutex_);
+    if (applyRing_.p) cudaStreamSynchronize(stream_);
+    applyRing_.Release();
 }
 
 void* Helmholtz::Scratch(size_t bytes) {
@@ -1436,14 +1443,27 @@ void Helmholtz::MultiplySlab(const z64* X, z64* Y, const z64* Bv, int k, int zFi
     CUDA_CHECK(cudaStreamSynchronize(stream_));
 }
 
+// Memory that MultiplyDevice keeps between calls (an allocation takes 1 to 30 ms,
+// the launches of a 400 MB grid 0.3 ms); more than that, where a single plane
+// is larger than a third of it, is freed again.
+constexpr size_t kKeptApplyRing = size_t(1) << 30;
+
 void Helmholtz::MultiplyDevice(z64* B, int k) {
     if (!dVel_.p) throw PspError(kNotInitialized, "DistHelmholtz is not initialized");
     CUDA_CHECK(cudaSetDevice(device_));
-    const int64_t nk = NumUnknowns() * k;
-    DeviceBuffer tmp;
-    tmp.Allocate(nk * sizeof(z64));
-    LaunchHelmholtzApply(B, tmp.as<z64>(), nullptr, dVel_.as<double>(), sp_, k, stream_);
-    CUDA_CHECK(cudaMemcpyAsync(B, tmp.p, nk * sizeof(z64), cudaMemcpyDeviceToDevice, stream_));
+    {
+        std::lock_guard<std::mutex> lock(applyMutex_);
+        const size_t need = InPlaceApplyBytes(sp_, k);
+        if (need > applyRing_.bytes) {
+            applyRing_.Release();
+            applyRing_.Allocate(need);
+        }
+        LaunchHelmholtzInPlace(B, applyRing_.p, dVel_.as<double>(), sp_, k, stream_);
+        if (applyRing_.bytes > kKeptApplyRing) {
+            CUDA_CHECK(cudaStreamSynchronize(stream_));
+            applyRing_.Release();
+        }
+    }
     CUDA_CHECK(cudaStreamSynchronize(stream_));
 }
 

@@ -4,6 +4,7 @@
 #include <complex>
 #include <cstring>
 #include <memory>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -206,6 +207,12 @@ private:
     std::unique_ptr<FactorStore<double>> f64_;
     std::unique_ptr<FactorStore<float>> f32_;
     DeviceBuffer pool_;
+    // planes of MultiplyDevice between its two steps, kept for the next call
+    // (its launches are queued under the mutex: callers on other threads share
+    // them and the stream's order)
+    DeviceBuffer applyRing_;
+    std::mutex applyMutex_;
+    void ReleaseApplyRing();
     // GMRES workspace, carved from pool_ by EnsureWorkspace
     z64 *wsX_ = nullptr, *wsX0_ = nullptr, *wsW_ = nullptr, *wsB_ = nullptr, *wsV_ = nullptr;
     z64 *wsCols_ = nullptr, *wsY_ = nullptr;
