@@ -66,14 +66,12 @@ struct GemmTile {
     int op, tm, tn;
 };
 
-enum GemmShape { kGemmSquare = 0, kGemmSkinny = 1 };
-int GemmTileM(GemmShape s);
-int GemmTileN(GemmShape s);
 // Appends the output tiles of `op` (index opIndex) to `tiles`.
 template <typename R>
-void AppendGemmTiles(const GemmOp<R>& op, int opIndex, GemmShape shape, std::vector<GemmTile>& tiles);
+void AppendGemmTiles(const GemmOp<R>& op, int opIndex, std::vector<GemmTile>& tiles);
 template <typename R>
-void LaunchGemm(const GemmOp<R>* ops, const GemmTile* tiles, int numTiles, GemmShape shape, cudaStream_t st);
+void LaunchGemm(const GemmOp<R>* ops, const GemmTile* tiles, int numTiles, cudaStream_t st);
+void PrepareGemmKernels();  // launch attributes (the current device's)
 
 // Tensor-core (tcgen05, split TF32) form of the complex-single batched GEMM
 // (factor_tc.cu) for ops with real alpha and beta: same op semantics, 128 x

@@ -143,6 +143,7 @@ class FactorStore {
 public:
     explicit FactorStore(Helmholtz& h) : h_(h), an_(h.an_) {
         PrepareFlowKernels<R>();
+        PrepareGemmKernels();
         // Complex-single factors use the tensor-core sweep from
         // kFlowTcMinCols right-hand sides on, unless the environment asks for
         // the CUDA cores (for comparisons).
@@ -623,7 +624,7 @@ std::unique_ptr<typename FactorStore<R>::FactorProgram> FactorStore<R>::FactorGr
                 return;
             }
         }
-        AppendGemmTiles(op, i, kGemmSquare, cc);
+        AppendGemmTiles(op, i, cc);
     };
     auto addOp = [&](const GemmOp<R>& op) {
         route(op, (int)ops.size(), tiles, tilesTc);
@@ -793,7 +794,7 @@ void FactorStore<R>::RunProgram(FactorProgram& pg, bool sync) {
             case Step::kGemm: {
                 ProfScope ps(st, kProfFactorGemm, s.flops, s.abytes);
                 const GemmOp<R>* ops = arenaTasks.At<GemmOp<R>>(s.a);
-                if (s.n) LaunchGemm<R>(ops, arenaTasks.At<GemmTile>(s.b), s.n, kGemmSquare, st);
+                if (s.n) LaunchGemm<R>(ops, arenaTasks.At<GemmTile>(s.b), s.n, st);
                 if constexpr (std::is_same<R, float>::value) {
                     if (s.nTc) LaunchGemmTc(arenaTasks.At<GemmTcTile>(s.c), s.nTc, status_.as<int>(), st);
                 }
