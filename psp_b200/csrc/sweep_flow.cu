@@ -47,8 +47,8 @@
 // twice per level and direction.  Stages and tiles hold 16 KB so that two CTAs
 // of five slots fit on an SM.  Measured against one launch per level and
 // direction with gathers between (sweeps of the whole preconditioner): FP64
-// 57 x 53 x 61, k = 5: 12.8 -> 6.9 ms (0.73 TB/s of factors); complex single
-// 75 x 67 x 58, k = 1: 8.4 -> 3.6 ms; 96 x 96 x 76, k = 1: 18.9 -> 7.5 ms
+// 57 x 53 x 61, k = 5: 12.8 -> 6.8 ms (0.74 TB/s of factors); complex single
+// 75 x 67 x 58, k = 1: 8.4 -> 3.5 ms; 96 x 96 x 76, k = 1: 18.9 -> 7.5 ms
 // (2.8 TB/s).
 #include <algorithm>
 
@@ -451,48 +451,53 @@ __device__ __forceinline__ void StageProduct(const unsigned char* slot, const un
 template <typename R, int NC, bool kBwd>
 __device__ __forceinline__ void StoreTile(const FlowTile& t, const FlowFront<R>& f, const cpx<R>* dinv, const int* idx,
                                           int k, int wrow, int rg, int cg,
-                                          const Acc<R> (&acc)[Cfg<R, NC>::RPT][Cfg<R, NC>::CPT], z64* B,
-                                          const PanelIO& io, const FlowWork& w) {
+                                          const Acc<R> (&acc)[Cfg<R, NC>::RPT][Cfg<R, NC>::CPT],
+                                          const FlowWork& w) {
     using C = Cfg<R, NC>;
-    // what the tile and the front say is read into registers first, and a
-    // backward tile's grid entries are loaded before any is written
     const int left = (kBwd ? f.s : f.s + f.u) - t.row0, pivots = f.s - t.row0, col0 = t.col0 + cg;
-    if (!kBwd) {
-        cpx<R>* const W = static_cast<cpx<R>*>(w.w) + (int64_t)(f.ndOff + t.row0) * k;
-        cpx<R>* const Pp = f.Pp;
+    cpx<R>* const own = static_cast<cpx<R>*>(kBwd ? w.x : w.w) + (int64_t)(f.ndOff + t.row0) * k;
+    cpx<R>* const Pp = f.Pp;
 #pragma unroll
-        for (int i = 0; i < C::RPT; ++i) {
-            const int row = wrow + RowIn<R, NC, kBwd>(i, rg);
-            const bool pivot = row < pivots;
-            cpx<R>* dst = pivot ? W + row * k : Pp + (int64_t)idx[row] * k;
-            const cpx<R> d = pivot ? dinv[row] : mk<R>(1, 0);
+    for (int i = 0; i < C::RPT; ++i) {
+        const int row = wrow + RowIn<R, NC, kBwd>(i, rg);
+        const bool pivot = kBwd || row < pivots;
+        cpx<R>* dst = pivot ? own + row * k : Pp + (int64_t)idx[row] * k;
+        const cpx<R> d = !kBwd && pivot ? dinv[row] : mk<R>(1, 0);
 #pragma unroll
-            for (int j = 0; j < C::CPT; ++j) {
-                const cpx<R> v = acc[i][j].Get();
-                if (row < left && col0 + j * C::CG < k) dst[col0 + j * C::CG] = pivot ? v * d : v;
-            }
+        for (int j = 0; j < C::CPT; ++j) {
+            const cpx<R> v = acc[i][j].Get();
+            if (row < left && col0 + j * C::CG < k) dst[col0 + j * C::CG] = !kBwd && pivot ? v * d : v;
         }
-    } else {
-        cpx<R>* const X = static_cast<cpx<R>*>(w.x) + (int64_t)(f.ndOff + t.row0) * k;
-        const bool accumulate = io.outAccumulate;
-        const int64_t ldk = io.ldk;
+    }
+}
+
+// The grid's entries of a backward tile, after the solution that other tiles
+// wait for has been released.  An entry is written once per launch, so an
+// addition that does not return is the same as one that does; loaded, added to
+// and stored before the release they made each backward level 1 us longer.
+template <typename R, int NC>
+__device__ __forceinline__ void StoreGrid(const FlowTile& t, const FlowFront<R>& f, const int* idx, int k, int wrow, int rg,
+                                          int cg, const Acc<R> (&acc)[Cfg<R, NC>::RPT][Cfg<R, NC>::CPT], z64* B,
+                                          const PanelIO& io) {
+    using C = Cfg<R, NC>;
+    const int left = f.s - t.row0, col0 = t.col0 + cg;
+    const bool accumulate = io.outAccumulate;
+    const int64_t ldk = io.ldk;
 #pragma unroll
-        for (int i = 0; i < C::RPT; ++i) {
-            const int row = wrow + RowIn<R, NC, kBwd>(i, rg);
-            const int at = row < left ? idx[row] : -1;
-            z64* const dst = B + at * ldk;
-            z64 old[C::CPT];
+    for (int i = 0; i < C::RPT; ++i) {
+        const int row = wrow + RowIn<R, NC, true>(i, rg);
+        const int at = row < left ? idx[row] : -1;
+        z64* const dst = B + at * ldk;
 #pragma unroll
-            for (int j = 0; j < C::CPT; ++j) {
-                old[j] = mk(0.0, 0.0);
-                if (accumulate && at >= 0 && col0 + j * C::CG < k) old[j] = dst[col0 + j * C::CG];
-            }
-#pragma unroll
-            for (int j = 0; j < C::CPT; ++j) {
-                const int col = col0 + j * C::CG;
-                const cpx<R> v = acc[i][j].Get();
-                if (row < left && col < k) X[row * k + col] = v;
-                if (at >= 0 && col < k) dst[col] = accumulate ? old[j] + ccast<double>(v) : ccast<double>(v);
+        for (int j = 0; j < C::CPT; ++j) {
+            const int col = col0 + j * C::CG;
+            if (at < 0 || col >= k) continue;
+            const z64 v = ccast<double>(acc[i][j].Get());
+            if (accumulate) {
+                asm volatile("red.relaxed.gpu.global.add.f64 [%0], %1;" ::"l"(&dst[col].re), "d"(v.re) : "memory");
+                asm volatile("red.relaxed.gpu.global.add.f64 [%0], %1;" ::"l"(&dst[col].im), "d"(v.im) : "memory");
+            } else {
+                dst[col] = v;
             }
         }
     }
@@ -625,9 +630,12 @@ __device__ __forceinline__ bool ComputeTile(const FlowTile& t, const FlowFront<R
             }
         }
     }
-    if (finish && kg == 0) StoreTile<R, NC, kBwd>(t, f, S.dinv[qs], S.idx[qs], k, wrow, rg, cg, acc, B, io, w);
+    if (finish && kg == 0) StoreTile<R, NC, kBwd>(t, f, S.dinv[qs], S.idx[qs], k, wrow, rg, cg, acc, w);
     umma::NamedBarrier(1, kComputeThreads);  // also: the reduction scratch and isLast are rewritten next
     if (finish && threadIdx.x == 0) AddRelease(w.done + t.signal);
+    if constexpr (kBwd) {
+        if (finish && kg == 0) StoreGrid<R, NC>(t, f, S.idx[qs], k, wrow, rg, cg, acc, B, io);
+    }
     return true;
 }
 
