@@ -4,7 +4,7 @@
 //   only r >= c when lowerC, the K range narrowed by the structural-zero
 //   flags (entries inside the range are read as stored).
 //
-// As in sweep_tc.cu, the complex product is one real product (A's rows as
+// As in sweep_flow_tc.cu, the complex product is one real product (A's rows as
 // interleaved (re, im) pairs, every B entry a 2x2 real block) and both
 // operands are split into tf32 head and tail; per 8-value K step
 //   A_hi B_hi + A_hi B_lo + A_lo B_hi   (three N = 128 MMAs, one accumulator)
@@ -14,18 +14,26 @@
 // Persistent and warp-specialized: CTA b takes tiles b, b + grid, ... (each
 // a 128 x 64 complex block described by one GemmTcTile record) and streams
 // their K stages (8 complex columns) through three roles:
-//   converters (8 warps)  asynchronous copies of operand stages into a
-//                         kRaw-slot ring kAhead stages ahead (zero-filled
-//                         outside the operands, any transposition), then the
-//                         split: A into TMEM (one lane per row), B into
-//                         one of two 64-byte-swizzled plane sets (d scales
-//                         B's rows here);
+//   converters (16 warps) two groups on alternating stages: asynchronous copies
+//                         of operand stages into a group's kRaw-slot ring kAhead
+//                         stages ahead (zero-filled outside the operands, any
+//                         transposition), then the split: A into TMEM (one lane
+//                         per row), B into one of four 64-byte-swizzled plane
+//                         sets (d scales B's rows here);
 //   MMA (one thread)      the split MMAs of a stage into one of two
-//                         128-column TMEM accumulators; stage flags mark
-//                         a tile's first and last stage;
-//   epilogue (4 warps)    one accumulator row per thread: alpha acc + beta C,
+//                         128-column TMEM accumulators; stage flags mark a
+//                         tile's last stage and a chain's first and last;
+//   epilogue (8 warps)    half an accumulator row per thread: alpha acc + beta C,
 //                         C staged in shared memory by copies issued while
-//                         the tile's MMAs run; coalesced column stores.
+//                         the tile's MMAs run (the next tile's as soon as eight
+//                         columns are read); coalesced column stores.
+//
+// What bounds it: a chain of waits per stage (copies, barrier, split, fences),
+// and at short K, which most fronts have (five to ten stages per tile), the
+// traffic and latency of C.  With one group of converters, four epilogue warps
+// and C copied between two barriers of a tile, the products of a 96^3 grid's
+// panels took 57.6 ms (42 TFLOP/s of complex single) and of a 140 x 140 x 80
+// grid's 241 ms; now 50.7 (48) and 213 ms (60).
 // Every wait is bounded; a timeout sets the value 2 in the status word and
 // ends all roles, leaving unfinished tiles unwritten.
 #include <climits>
@@ -39,11 +47,12 @@ namespace {
 
 constexpr int kBM = kGemmTcRows, kBN = kGemmTcCols;
 constexpr int kSK = 8;  // complex K per stage: one 64-byte plane row
-constexpr int kEpiThreads = 128, kConvThreads = 256;
-constexpr int kConv0 = kEpiThreads, kMma0 = kConv0 + kConvThreads;
+constexpr int kEpiThreads = 256;               // two threads per row, half of the columns each
+constexpr int kConvGroups = 2, kConvThreads = 256;  // converters per group
+constexpr int kConv0 = kEpiThreads, kMma0 = kConv0 + kConvGroups * kConvThreads;
 constexpr int kFThreads = kMma0 + 32;
-constexpr int kRaw = 6, kAhead = kRaw - 1;  // raw slots; stages in flight ahead of the conversion
-constexpr int kPlaneSets = 2, kAccs = 2;
+constexpr int kRaw = 3, kAhead = kRaw - 1;  // per group: raw slots; stages in flight ahead of the conversion
+constexpr int kPlaneSets = 2 * kConvGroups, kAccs = 2;
 
 constexpr uint32_t kBPl = 2 * kBN * 64;  // 8 KB: B' has 2 kBN rows of 16 tf32
 constexpr uint32_t kPlSet = 2 * kBPl;     // B hi, B lo
@@ -58,11 +67,11 @@ constexpr int kApad = kBM + 1, kBpad = kBN + 1;  // raw A [kc][row], raw B [kc][
 constexpr uint32_t kRawA = kSK * kApad * 8, kRawB = kSK * kBpad * 8;
 constexpr uint32_t kRawSlot = kRawA + kRawB + kSK * 8;  // + d
 constexpr uint32_t kRawOff = kPlaneSets * kPlSet;
-constexpr uint32_t kStageOff = kRawOff + kRaw * kRawSlot;  // C staging [col][row]
+constexpr uint32_t kStageOff = kRawOff + kConvGroups * kRaw * kRawSlot;  // C staging [col][row]
 constexpr size_t kFactorTcSmem = kStageOff + (size_t)kBN * kBM * 8 + 1024;
 constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kIdesc = umma::InstrDescTf32(kBM, 2 * kBN);
-constexpr int kFirst = 1, kLast = 2;  // stage flags: a tile's first and last stage
+constexpr int kLast = 2;  // stage flag: a tile's last stage
 // The tensor core adds each MMA's products into its FP32 accumulator with
 // truncation, so an accumulator holds at most kChainStages stages (64
 // complex K); the epilogue sums a tile's chains in FP32 (round to nearest)
@@ -81,8 +90,8 @@ struct Sync {
     uint64_t planeFull[kPlaneSets], planeEmpty[kPlaneSets];
     uint64_t accFull[kAccs], accEmpty[kAccs];
     uint64_t mmaDrain;           // the MMA thread's last commit when a role gave up
-    int rawFlags[kRaw];          // written and read by converter thread 0
-    int planeFlags[kPlaneSets];  // converter thread 0 -> MMA thread
+    int rawFlags[kConvGroups][kRaw];  // written and read by a group's thread 0
+    int planeFlags[kPlaneSets];  // converters -> MMA thread
     uint32_t tmem;
     int abort;
 };
@@ -201,58 +210,66 @@ __device__ __forceinline__ void ConvertStage(const unsigned char* raw, unsigned 
 }
 
 __device__ void ConverterRole(const GemmTcTile* tiles, int n, unsigned char* smem, Sync& S, int* status) {
-    const int ct = threadIdx.x - kConv0;
+    const int group = (threadIdx.x - kConv0) / kConvThreads, ct = (threadIdx.x - kConv0) % kConvThreads;
+    const int lane = threadIdx.x & 31, bar = group ? 3 : 1;
     const int G = gridDim.x;
-    unsigned char* raw = smem + kRawOff;
+    unsigned char* raw = smem + kRawOff + group * kRaw * kRawSlot;
     // load cursor: tile t (record cur), stage st of nst; the next record is
-    // read a tile ahead
-    int t = blockIdx.x, st = 0;
+    // read a tile ahead.  The group's stages are the CTA's stages group,
+    // group + 2, ...
+    int t = blockIdx.x, st = group;
     bool more = t < n;
     GemmTcTile cur, nxt;
     if (more) cur = tiles[t];
     if (t + G < n) nxt = tiles[t + G];
     int nst = more ? StagesOf(cur) : 0;
-    int issued = 0;
+    auto settle = [&]() {  // on to the tile that stage st lies in
+        while (more && st >= nst) {
+            st -= nst;
+            t += G;
+            more = t < n;
+            if (more) {
+                cur = nxt;
+                nst = StagesOf(cur);
+                if (t + G < n) nxt = tiles[t + G];
+            }
+        }
+    };
+    settle();
+    int issued = 0, in = 0;
     // one committed copy group per stage slot, empty past the stream's end
     auto issueNext = [&]() {
         if (more) {
-            const int slot = issued % kRaw;
-            IssueStage(cur, st, raw + slot * kRawSlot, ct);
+            IssueStage(cur, st, raw + in * kRawSlot, ct);
             if (ct == 0)
-                S.rawFlags[slot] = (st == 0 ? kFirst : 0) | (st == nst - 1 ? kLast : 0) |
-                                   (st % kChainStages == 0 ? kChainFirst : 0) |
-                                   (st % kChainStages == kChainStages - 1 || st == nst - 1 ? kChainLast : 0);
+                S.rawFlags[group][in] = (st == nst - 1 ? kLast : 0) | (st % kChainStages == 0 ? kChainFirst : 0) |
+                                        (st % kChainStages == kChainStages - 1 || st == nst - 1 ? kChainLast : 0);
             ++issued;
-            if (++st == nst) {
-                t += G;
-                st = 0;
-                more = t < n;
-                if (more) {
-                    cur = nxt;
-                    nst = StagesOf(cur);
-                    if (t + G < n) nxt = tiles[t + G];
-                }
-            }
+            if (++in == kRaw) in = 0;
+            st += kConvGroups;
+            settle();
         }
         umma::CpAsyncCommit();
     };
     for (int i = 0; i < kAhead; ++i) issueNext();
-    for (int g = 0; g < issued; ++g) {
-        const int p = g % kPlaneSets;
+    int slot = 0;
+    for (int l = 0; l < issued; ++l) {
+        const int g = kConvGroups * l + group, p = g % kPlaneSets;
         umma::CpAsyncWait<kAhead - 1>();
         bool ok = true;
         if (ct == 0 && g >= kPlaneSets) ok = Wait(&S.planeEmpty[p], ((g / kPlaneSets) - 1) & 1, S, status);
-        // stage g's copies are visible to every converter, stage g-1's slot
-        // is free, and plane set p is free (its MMAs completed)
-        if (umma::NamedBarrierOr(1, kConvThreads, !ok)) break;
-        const int slot = g % kRaw;
-        if (ct == 0) S.planeFlags[p] = S.rawFlags[slot];
+        // the stage's copies are visible to the whole group, the slot of its
+        // stage before is free, and plane set p is free (its MMAs completed)
+        if (umma::NamedBarrierOr(bar, kConvThreads, !ok)) break;
+        if (ct == 0) S.planeFlags[p] = S.rawFlags[group][slot];
         issueNext();
         ConvertStage(raw + slot * kRawSlot, smem + p * kPlSet, S.tmem + ACol(p), ct);
         umma::TmemStoreWait();
         umma::FenceProxyAsync();
         umma::FenceBeforeSync();
-        umma::MbarArrive(&S.planeFull[p]);
+        __syncwarp();
+        if (lane == 0) umma::MbarArrive(&S.planeFull[p]);
+        if (++slot == kRaw) slot = 0;
     }
     umma::CpAsyncWaitAll();
 }
@@ -290,24 +307,26 @@ __device__ void MmaRole(int n, unsigned char* smem, Sync& S, int* status) {
 
 // ------------------------------------------------------------------ epilogue
 
-// This thread's copies of its row of the C tile into the staging tile
-// ([col][row]), where the tile writes and beta is nonzero.
-__device__ __forceinline__ void IssueC(const GemmTcTile& T, c32* stage) {
-    const int r = threadIdx.x;
+constexpr int kSub = 8;                  // columns of the write-out at a time
+constexpr int kChunks = kBN / 2 / kSub;  // of a thread's half row
+
+// This thread's copies of kSub columns from c0 of its row of the C tile into
+// the staging tile ([col][row]; no other thread uses these entries), where the
+// tile writes and beta is nonzero.
+__device__ __forceinline__ void IssueC(const GemmTcTile& T, c32* stage, int r, int c0) {
     if (T.beta == 0.f || r >= T.m) return;
-    const int ncol = min(T.n, r - T.diag + 1);  // r - c >= diag
-    const c32* src = T.C + r;
-    for (int c = 0; c < ncol; ++c, src += T.ldc) umma::CpAsync8(stage + c * kBM + r, src, 8u);
+    const int c1 = min(min(T.n, r - T.diag + 1), c0 + kSub);  // r - c >= diag
+    const c32* src = T.C + r + (int64_t)c0 * T.ldc;
+    for (int c = c0; c < c1; ++c, src += T.ldc) umma::CpAsync8(stage + c * kBM + r, src, 8u);
 }
 
-// alpha acc + beta C for this thread's row of 16 columns from column j0.
+// alpha acc + beta C for this thread's row of kSub columns from column j0.
 template <bool kFull>
-__device__ __forceinline__ void StoreCols(const GemmTcTile& T, const float (&v)[32], const c32* stage, int j0) {
-    const int r = threadIdx.x;
+__device__ __forceinline__ void StoreCols(const GemmTcTile& T, const float (&v)[2 * kSub], const c32* stage, int r, int j0) {
     c32* dst = T.C + r + (int64_t)j0 * T.ldc;
     const float al = T.alpha, be = T.beta;
 #pragma unroll
-    for (int q = 0; q < 16; ++q, dst += T.ldc) {
+    for (int q = 0; q < kSub; ++q, dst += T.ldc) {
         const int c = j0 + q;
         if (!kFull && (r >= T.m || c >= T.n || r - c < T.diag)) continue;
         c32 out = mk(al * v[2 * q], al * v[2 * q + 1]);
@@ -320,80 +339,82 @@ __device__ __forceinline__ void StoreCols(const GemmTcTile& T, const float (&v)[
     }
 }
 
+// A wait of the whole warp, with one answer.
+__device__ __forceinline__ bool WaitAll(uint64_t* mbar, uint32_t parity, Sync& S, int* status) {
+    return __all_sync(~0u, Wait(mbar, parity, S, status));
+}
+
+// No thread needs another's entries, so warps go on by themselves; the next
+// tile's C is on its way as soon as a chunk's place is free.
 __device__ void EpilogueRole(const GemmTcTile* tiles, int n, c32* stage, Sync& S, int* status) {
-    const int tid = threadIdx.x, warp = tid / 32;
+    const int row = threadIdx.x % kBM, c0 = threadIdx.x / kBM * (kBN / 2);
     const int G = gridDim.x;
-    const uint32_t lane = (uint32_t)(warp * 32) << 16;
+    const uint32_t lane = (uint32_t)(row & ~31) << 16;
     GemmTcTile cur;
-    if ((int)blockIdx.x < n) {
-        cur = tiles[blockIdx.x];
-        IssueC(cur, stage);
+    if ((int)blockIdx.x < n) cur = tiles[blockIdx.x];
+    for (int j = 0; j < kChunks; ++j) {
+        if ((int)blockIdx.x < n) IssueC(cur, stage, row, c0 + kSub * j);
+        umma::CpAsyncCommit();
     }
-    umma::CpAsyncCommit();
-    const uint32_t tsum = S.tmem + lane + kSumCol;
+    const uint32_t tsum = S.tmem + lane + kSumCol + 2 * c0;
     int q = 0;  // chains drained
     for (int t = blockIdx.x; t < n; t += G) {
         GemmTcTile nxt;
-        if (t + G < n) nxt = tiles[t + G];
-        // every chain but the last goes into the sum region; every epilogue
-        // thread takes the same branches (they share named barriers)
+        const bool more = t + G < n;
+        if (more) nxt = tiles[t + G];
+        // every chain but the last goes into the sum region
         const int nch = (StagesOf(cur) + kChainStages - 1) / kChainStages;
-        bool quit = false;  // the same on every epilogue thread
-        for (int c = 0; c + 1 < nch && !quit; ++c, ++q) {
+        bool ok = true;
+        for (int c = 0; c + 1 < nch; ++c, ++q) {
             const int a = q % kAccs;
-            const bool ok = Wait(&S.accFull[a], (q / kAccs) & 1, S, status);
-            quit = umma::NamedBarrierOr(2, kEpiThreads, !ok);
-            if (quit) break;
+            ok = WaitAll(&S.accFull[a], (q / kAccs) & 1, S, status);
+            if (!ok) break;
             umma::FenceAfterSync();
-            const uint32_t acc = S.tmem + lane + a * kAccCols;
+            const uint32_t acc = S.tmem + lane + a * kAccCols + 2 * c0;
 #pragma unroll 1
-            for (int j = 0; j < kBN / 16; ++j) {
-                float v[32];
-                umma::TmemLoad32(acc + 32 * j, v);
+            for (int j = 0; j < kChunks; ++j) {
+                float v[2 * kSub];
+                umma::TmemLoad16(acc + 2 * kSub * j, v);
                 if (c > 0) {
-                    float w[32];
-                    umma::TmemLoad32(tsum + 32 * j, w);
+                    float w[2 * kSub];
+                    umma::TmemLoad16(tsum + 2 * kSub * j, w);
 #pragma unroll
-                    for (int e = 0; e < 32; ++e) v[e] += w[e];
+                    for (int e = 0; e < 2 * kSub; ++e) v[e] += w[e];
                 }
-                umma::TmemStore32NoWait(tsum + 32 * j, v);
+                umma::TmemStore16(tsum + 2 * kSub * j, v);
             }
             umma::TmemStoreWait();
             umma::FenceBeforeSync();
             umma::MbarArrive(&S.accEmpty[a]);
         }
-        if (quit) break;
         const int a = q % kAccs;
-        const bool ok = Wait(&S.accFull[a], (q / kAccs) & 1, S, status);
+        if (!ok || !WaitAll(&S.accFull[a], (q / kAccs) & 1, S, status)) break;
         ++q;
-        umma::CpAsyncWaitAll();
-        if (umma::NamedBarrierOr(2, kEpiThreads, !ok)) break;  // the staged C is visible
         umma::FenceAfterSync();
         const bool full = cur.m == kBM && cur.n == kBN && cur.diag <= 1 - kBN;
-        const uint32_t acc = S.tmem + lane + a * kAccCols;
+        const uint32_t acc = S.tmem + lane + a * kAccCols + 2 * c0;
 #pragma unroll 1
-        for (int j = 0; j < kBN / 16; ++j) {
-            float v[32];
-            umma::TmemLoad32(acc + 32 * j, v);
+        for (int j = 0; j < kChunks; ++j) {
+            float v[2 * kSub];
+            umma::TmemLoad16(acc + 2 * kSub * j, v);
             if (nch > 1) {
-                float w[32];
-                umma::TmemLoad32(tsum + 32 * j, w);
+                float w[2 * kSub];
+                umma::TmemLoad16(tsum + 2 * kSub * j, w);
 #pragma unroll
-                for (int e = 0; e < 32; ++e) v[e] += w[e];
+                for (int e = 0; e < 2 * kSub; ++e) v[e] += w[e];
             }
+            umma::CpAsyncWait<kChunks - 1>();  // this chunk of C
             if (full)
-                StoreCols<true>(cur, v, stage, 16 * j);
+                StoreCols<true>(cur, v, stage, row, c0 + kSub * j);
             else
-                StoreCols<false>(cur, v, stage, 16 * j);
+                StoreCols<false>(cur, v, stage, row, c0 + kSub * j);
+            __syncwarp();
+            if (more) IssueC(nxt, stage, row, c0 + kSub * j);
+            umma::CpAsyncCommit();
         }
         umma::FenceBeforeSync();
         umma::MbarArrive(&S.accEmpty[a]);
-        umma::NamedBarrier(2, kEpiThreads);  // the staging tile is rewritten next
-        if (t + G < n) {
-            cur = nxt;
-            IssueC(cur, stage);
-        }
-        umma::CpAsyncCommit();
+        if (more) cur = nxt;
     }
     umma::CpAsyncWaitAll();
 }
@@ -409,7 +430,7 @@ __global__ void __launch_bounds__(kFThreads, 1)
     const int tid = threadIdx.x;
     if (tid == 0) {
         for (int i = 0; i < kPlaneSets; ++i) {
-            umma::MbarInit(&S.planeFull[i], kConvThreads);
+            umma::MbarInit(&S.planeFull[i], kConvThreads / 32);
             umma::MbarInit(&S.planeEmpty[i], 1);
         }
         for (int i = 0; i < kAccs; ++i) {
