@@ -37,9 +37,9 @@
 // hand sides loaded through registers a stage took 0.85 us, with the children's
 // updates and the grid written on the way out a tile's write-out took 5 us
 // instead of 3, and with tickets taken two tiles ahead the narrow levels were
-// badly balanced (39 instead of 29 ms per sweep at 116^3).  Measured against one
-// launch per level and direction, whole sweeps: 116^3, k = 16: 44.1 -> 29.0 ms
-// (1.8 TB/s of factors); 96 x 96 x 76, k = 32: 34.7 -> 18.7 ms.
+// badly balanced (39 instead of 29 ms then per sweep at 116^3).  Measured against one
+// launch per level and direction, whole sweeps: 116^3, k = 16: 44.1 -> 27.2 ms
+// (1.9 TB/s of factors); 96 x 96 x 76, k = 32: 34.7 -> 16.9 ms.
 #include <algorithm>
 
 #include "sweep_flow.cuh"
@@ -477,7 +477,32 @@ __device__ __forceinline__ void LoadSums(uint32_t taddr, uint32_t tsum, bool add
     for (int c = 0; c < kSub; ++c) acc[c] = mk(a[2 * c], a[2 * c + 1]);
 }
 
-__device__ __forceinline__ void StoreRow(c32* dst, const c32 (&v)[kSub], int n, bool pair) {
+// 32-byte accesses of four columns (k a multiple of 4: rows of whole 32-byte
+// sectors).  A lane's row is a line of its own, so every access costs a request
+// of its own: with 16-byte ones the children's rows and the write-out held up
+// the loads of all other roles at the wide levels (116^3, k = 16: 28.8 -> 27.2 ms
+// per sweep; 96 x 96 x 76, k = 32: 18.5 -> 17.0 ms; 140^2, k = 32 solve 401 -> 376 ms).
+__device__ __forceinline__ void Store4(c32* dst, const c32* v) {
+    asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(dst), "f"(v[0].re), "f"(v[0].im), "f"(v[1].re),
+                 "f"(v[1].im), "f"(v[2].re), "f"(v[2].im), "f"(v[3].re), "f"(v[3].im)
+                 : "memory");
+}
+__device__ __forceinline__ void Load4(c32* v, const c32* src) {
+    asm volatile("ld.global.L1::no_allocate.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=f"(v[0].re), "=f"(v[0].im), "=f"(v[1].re), "=f"(v[1].im), "=f"(v[2].re), "=f"(v[2].im), "=f"(v[3].re),
+                   "=f"(v[3].im)
+                 : "l"(src)
+                 : "memory");
+}
+
+__device__ __forceinline__ void StoreRow(c32* dst, const c32 (&v)[kSub], int n, int align) {
+    if (align == 4) {
+#pragma unroll
+        for (int j = 0; j < kSub; j += 4)
+            if (j < n) Store4(dst + j, v + j);
+        return;
+    }
+    const bool pair = align == 2;
 #pragma unroll
     for (int j = 0; j < kSub; j += 2) {
         if (pair) {
@@ -499,18 +524,39 @@ struct RowOut {
 };
 
 // Writes columns col .. col + n - 1 of the row.
-__device__ __forceinline__ void WriteRow(const RowOut& o, int col, int n, bool pair, c32 (&acc)[kSub]) {
+__device__ __forceinline__ void WriteRow(const RowOut& o, int col, int n, int align, c32 (&acc)[kSub]) {
     if (!o.dst) return;
     if (o.pivot) {
 #pragma unroll
         for (int j = 0; j < kSub; ++j) acc[j] = acc[j] * o.dinv;
     }
-    StoreRow(o.dst + col, acc, n, pair);
+    StoreRow(o.dst + col, acc, n, align);
 }
 
 // The same columns of the grid (+)= acc.  A grid entry is written once per
 // launch, so an addition that does not return is the same as one that does.
-__device__ __forceinline__ void WriteGrid(z64* dst, int n, bool accumulate, const c32 (&acc)[kSub]) {
+// Two columns (32 bytes) at a time where the rows are aligned for it (`wide`): a
+// lane's row is far from its neighbours', and eight-byte additions ask L2 four
+// times as often.  With 16 columns per tile the loads' latency costs more than
+// that (116^3: 27.6 instead of 27.2 ms); with 32 it is 16.9 instead of 17.0 ms.
+__device__ __forceinline__ void WriteGrid(z64* dst, int n, bool accumulate, bool wide, const c32 (&acc)[kSub]) {
+    if (wide) {
+        double v[kSub][2];
+#pragma unroll
+        for (int j = 0; j < kSub; j += 2) {
+            v[j][0] = v[j][1] = v[j + 1][0] = v[j + 1][1] = 0;
+            if (accumulate && j < n)
+                asm volatile("ld.global.L1::no_allocate.v4.f64 {%0,%1,%2,%3}, [%4];"
+                             : "=d"(v[j][0]), "=d"(v[j][1]), "=d"(v[j + 1][0]), "=d"(v[j + 1][1]) : "l"(dst + j) : "memory");
+        }
+#pragma unroll
+        for (int j = 0; j < kSub; j += 2)
+            if (j < n)
+                asm volatile("st.global.v4.f64 [%0], {%1,%2,%3,%4};" ::"l"(dst + j), "d"(v[j][0] + acc[j].re),
+                             "d"(v[j][1] + acc[j].im), "d"(v[j + 1][0] + acc[j + 1].re), "d"(v[j + 1][1] + acc[j + 1].im)
+                             : "memory");
+        return;
+    }
 #pragma unroll
     for (int j = 0; j < kSub; ++j) {
         if (j >= n) break;
@@ -545,6 +591,8 @@ __device__ void EpilogueRole(int k, Sync& S, z64* B, const PanelIO& io, const Fl
     const uint32_t lanes = (uint32_t)(row & ~31) << 16;
     const uint32_t tsum = S.tmem + C::kSumCol + group * 2 * NC + lanes;
     const bool pair = (k & 1) == 0, accumulate = io.outAccumulate;
+    const int align = k % 4 == 0 ? 4 : pair ? 2 : 1;  // columns of an aligned access
+    const bool wide = NC == 32 && pair && io.ldk % 2 == 0 && (reinterpret_cast<uintptr_t>(B) & 31) == 0;
     int c = 0, own = 0;  // chains of all tiles, and of this group's
     for (int q = 0;; ++q) {
         const int qs = q % kQueue;
@@ -592,17 +640,31 @@ __device__ void EpilogueRole(int k, Sync& S, z64* B, const PanelIO& io, const Fl
                     const c32* c1 = in && f.P1 ? f.P1 + (int64_t)r * k + col0 : nullptr;
 #pragma unroll 1
                     for (int h = 0; h < NC / kSub; ++h) {
-                        Unit<float, 2> a[kSub / 2], b[kSub / 2];
-#pragma unroll
-                        for (int j = 0; j < kSub / 2; ++j) {
-                            const int n = h * kSub + 2 * j;
-                            a[j] = b[j] = ZeroUnit<float, 2>();
-                            if (c0 && n < ncol) LoadUnit<float, 2>(a[j], c0 + n, pair, n + 1 < ncol);
-                            if (c1 && n < ncol) LoadUnit<float, 2>(b[j], c1 + n, pair, n + 1 < ncol);
-                        }
                         c32 v[kSub];
+                        if (align == 4) {
+                            c32 a[kSub], b[kSub];
 #pragma unroll
-                        for (int j = 0; j < kSub; ++j) v[j] = a[j / 2].z[j % 2] + b[j / 2].z[j % 2];
+                            for (int j = 0; j < kSub; ++j) a[j] = b[j] = mk(0.f, 0.f);
+#pragma unroll
+                            for (int j = 0; j < kSub; j += 4) {
+                                const int n = h * kSub + j;
+                                if (c0 && n < ncol) Load4(a + j, c0 + n);
+                                if (c1 && n < ncol) Load4(b + j, c1 + n);
+                            }
+#pragma unroll
+                            for (int j = 0; j < kSub; ++j) v[j] = a[j] + b[j];
+                        } else {
+                            Unit<float, 2> a[kSub / 2], b[kSub / 2];
+#pragma unroll
+                            for (int j = 0; j < kSub / 2; ++j) {
+                                const int n = h * kSub + 2 * j;
+                                a[j] = b[j] = ZeroUnit<float, 2>();
+                                if (c0 && n < ncol) LoadUnit<float, 2>(a[j], c0 + n, pair, n + 1 < ncol);
+                                if (c1 && n < ncol) LoadUnit<float, 2>(b[j], c1 + n, pair, n + 1 < ncol);
+                            }
+#pragma unroll
+                            for (int j = 0; j < kSub; ++j) v[j] = a[j / 2].z[j % 2] + b[j / 2].z[j % 2];
+                        }
                         StoreSums(tsum, h, v);
                     }
                     umma::TmemStoreWait();
@@ -654,7 +716,7 @@ __device__ void EpilogueRole(int k, Sync& S, z64* B, const PanelIO& io, const Fl
                 for (int n = 0; n < kSub; n += 2)
                     mine[n / 2 * kRows] = make_float4(acc[n].re, acc[n].im, acc[n + 1].re, acc[n + 1].im);
             } else {
-                WriteRow(o, col0 + h * kSub, ncol - h * kSub, pair, acc);
+                WriteRow(o, col0 + h * kSub, ncol - h * kSub, align, acc);
             }
         }
         if (nsplit > 1) {
@@ -692,7 +754,7 @@ __device__ void EpilogueRole(int k, Sync& S, z64* B, const PanelIO& io, const Fl
                             }
                     }
                     if (bwd) StoreSums(tsum, h, acc);
-                    WriteRow(o, col0 + h * kSub, ncol - h * kSub, pair, acc);
+                    WriteRow(o, col0 + h * kSub, ncol - h * kSub, align, acc);
                 }
             }
         }
@@ -708,7 +770,7 @@ __device__ void EpilogueRole(int k, Sync& S, z64* B, const PanelIO& io, const Fl
                 c32 acc[kSub];
 #pragma unroll
                 for (int j = 0; j < kSub; ++j) acc[j] = mk(a[2 * j], a[2 * j + 1]);
-                if (o.grid) WriteGrid(o.grid + col0 + h * kSub, ncol - h * kSub, accumulate, acc);
+                if (o.grid) WriteGrid(o.grid + col0 + h * kSub, ncol - h * kSub, accumulate, wide, acc);
             }
         }
         __syncwarp();
