@@ -126,8 +126,9 @@ int psp_cu_precondition_device(psp_cu_handle* h, double* d_B, int k);
  * counterpart in the reference: it exists for callers that cannot allocate
  * while they call -- code running inside its own CUDA stream capture, where an
  * allocation breaks the capture, and services that reserve all device memory
- * up front.  psp_cu_multiply_device allocates its nx*ny*nz*k temporary on
- * every call; this variant uses a 16 MiB file-scope device array instead, so
+ * up front.  psp_cu_multiply_device keeps its temporary (nx*ny*nz*k entries, at
+ * most 1 GiB) with the handle until psp_cu_finalize and allocates when a call
+ * needs more than is kept; this variant uses a 16 MiB file-scope device array instead, so
  * nx*ny*nz*k must not exceed 1048576 (PSP_CU_LOGIC_ERROR otherwise).  The
  * first call on a device looks up that array's device address; make it before
  * any stream capture.  All calls share the array: calls that overlap on the

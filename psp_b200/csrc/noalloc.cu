@@ -1,9 +1,9 @@
 // B := A B without any device allocation (psp_cu_multiply_device_noalloc).
 //
 // The in-place operator apply needs a full-size temporary for A B before it
-// can overwrite B.  psp_cu_multiply_device allocates that temporary on every
-// call; this variant keeps it in a file-scope device array instead, so the
-// call itself never allocates.  It serves callers that cannot allocate device
+// can overwrite B.  psp_cu_multiply_device allocates that temporary when a call
+// needs more than its handle has kept; this variant keeps it in a file-scope
+// device array instead, so the call itself never allocates.  It serves callers that cannot allocate device
 // memory at the time they call: code that runs while one of its own streams
 // is being captured into a CUDA graph (an allocation there invalidates or
 // breaks the capture), and services that reserve all device memory at
