@@ -110,7 +110,7 @@ struct Sync {
     uint64_t tma[kMaxSlots], empty[kMaxSlots];
     uint64_t rhs[kMaxChunks], rhsEmpty[kMaxChunks];
     uint64_t tileFull[kQueue], tileEmpty[kQueue];
-    int abort, isLast, lastCta;
+    int abort, isLast, lastCta, issued;
 };
 
 // A right-hand-side entry in a chunk: complex single as (re, re, im, im), the
@@ -133,11 +133,10 @@ __device__ void ProducerRole(const FlowFront<R>* __restrict__ fr, const FlowTile
     asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
     TileSource<R> src;
     src.Start(fr, tiles, n, w.ctrl, false);
-    int g = 0, issued = 0;
-    bool ok = true;
+    int g = 0;
     for (int q = 0;; ++q) {
         const int qs = q % kQueue;
-        if (q >= kQueue && !WaitWarp(&S.tileEmpty[qs], ((q / kQueue) - 1) & 1, S, w.status)) { ok = false; break; }
+        if (q >= kQueue && !WaitWarp(&S.tileEmpty[qs], ((q / kQueue) - 1) & 1, S, w.status)) return;
         if (lane < kCtxWords) reinterpret_cast<int4*>(&S.queue[qs])[lane] = src.ctx;
         __syncwarp();
         if (lane == 0) umma::MbarArrive(&S.tileFull[qs]);
@@ -147,7 +146,7 @@ __device__ void ProducerRole(const FlowFront<R>* __restrict__ fr, const FlowTile
         const int nst = t.nst;
         for (int st = 0; st < nst; ++st, ++g) {
             const int slot = g % C::kSlots;
-            if (g >= C::kSlots && !WaitWarp(&S.empty[slot], ((g / C::kSlots) - 1) & 1, S, w.status)) { ok = false; break; }
+            if (g >= C::kSlots && !WaitWarp(&S.empty[slot], ((g / C::kSlots) - 1) & 1, S, w.status)) return;
             if (lane == 0) {
                 unsigned char* dst = smem + slot * kGBytes;
                 const int kBase = t.k0 + st * kStageK;
@@ -160,16 +159,11 @@ __device__ void ProducerRole(const FlowFront<R>* __restrict__ fr, const FlowTile
                     TmaLoadStream(dst, map, 2 * kBase, t.row0, &S.tma[slot], policy);
                     TmaLoadStream(dst + kGBytes / 2, map, 2 * kBase + kStageK, t.row0, &S.tma[slot], policy);
                 }
+                S.issued = g + 1;
             }
-            issued = g + 1;
             __syncwarp();
         }
-        if (!ok) break;
         src.Take();
-    }
-    if (!ok) {  // drain: the last copy into every slot has landed before the CTA exits
-        for (int s = 0; s < C::kSlots && s < issued; ++s)
-            umma::MbarWaitBounded(&S.tma[s], ((issued - 1 - s) / C::kSlots) & 1, nullptr);
     }
 }
 
@@ -684,6 +678,7 @@ __global__ void __launch_bounds__(kThreads, 2) sweep_flow_kernel(const FlowFront
             umma::MbarInit(&S.tileEmpty[i], kLoadWarps + kComputeWarps);
         }
         S.abort = 0;
+        S.issued = 0;
         umma::FenceMbarInit();
     }
     __syncthreads();
@@ -691,6 +686,13 @@ __global__ void __launch_bounds__(kThreads, 2) sweep_flow_kernel(const FlowFront
     else if (tid < kProd0) LoaderRole<R, NC>(k, smem, S, io, w);
     else ProducerRole<R, NC>(fr, tiles, n, smem, S, w);
     __syncthreads();
+    // Every role has returned.  When one gave up, copies that nobody waited for may
+    // be in flight, whether or not the producer was done: the last one into every
+    // slot lands (bounded) before the CTA exits.  S.abort is no longer written.
+    if (*reinterpret_cast<volatile int*>(&S.abort)) {
+        if (tid == kProd0) DrainCopies<C::kSlots>(S);
+        __syncthreads();
+    }
     LeaveFlow(w, &S.lastCta);
 }
 

@@ -177,6 +177,14 @@ struct TileSource {
     }
 };
 
+// After a role gave up: waits (bounded) until the last copy into each of the ring's
+// slots has landed, so none is in flight when the CTA exits.
+template <int kSlots, typename Sync>
+__device__ __forceinline__ void DrainCopies(Sync& S) {
+    for (int s = 0; s < kSlots && s < S.issued; ++s)
+        umma::MbarWaitBounded(&S.tma[s], ((S.issued - 1 - s) / kSlots) & 1, nullptr);
+}
+
 // At the end of a CTA: the last one leaves the ticket and the counters at zero.
 __device__ __forceinline__ void LeaveFlow(const FlowWork& w, int* lastCta) {
     if (threadIdx.x == 0) {

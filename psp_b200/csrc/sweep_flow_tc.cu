@@ -149,15 +149,6 @@ __device__ void ProducerRole(const FlowFront<float>* __restrict__ fr, const Flow
     }
 }
 
-// After a role gave up: waits (bounded) until the last copy into every slot
-// has landed, so none is in flight when the CTA exits.
-template <int NC>
-__device__ __forceinline__ void DrainCopies(Sync& S) {
-    constexpr int R = Cfg<NC>::kSlots;
-    for (int s = 0; s < R && s < S.issued; ++s)
-        umma::MbarWaitBounded(&S.tma[s], ((S.issued - 1 - s) / R) & 1, nullptr);
-}
-
 // ------------------------------------------------------------------ loaders
 
 __device__ __forceinline__ void Split2(c32 x, float2& hi, float2& lo) {
@@ -830,7 +821,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) sweep_flow_tc_kernel(const Flow
             if (ElectOne()) umma::CommitTo(&S.mmaDrain);
             umma::MbarWaitBounded(&S.mmaDrain, 0, nullptr);
         }
-        if (tid == kProd0) DrainCopies<NC>(S);
+        if (tid == kProd0) DrainCopies<C::kSlots>(S);
         umma::FenceBeforeSync();
         __syncthreads();
     }
