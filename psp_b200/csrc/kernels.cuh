@@ -218,7 +218,7 @@ struct FlowWork {
     int* done;       // finished tiles per front, forward then backward (zero between launches)
     int* ctrl;       // ticket, finished CTAs (zero between launches)
     int* status;     // bit 2: a wait timed out
-    int numDone;
+    int numDone, numCounters;
 };
 
 // Columns of a tile for k right-hand sides: the power of two that holds them, at most kFlowMaxCols.

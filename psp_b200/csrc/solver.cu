@@ -1047,6 +1047,7 @@ void FactorStore<R>::SolvePanel(z64* B, int ldk, int k, int p, int inMode, int o
     w.ctrl = P.done.template as<int>();
     w.done = w.ctrl + 2;
     w.numDone = 2 * nn_;
+    w.numCounters = (int)(P.counters.bytes / sizeof(int));
     w.status = status_.template as<int>();
     {
         ProfScope ps(st, kProfGatherScatter);

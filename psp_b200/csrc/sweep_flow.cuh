@@ -186,6 +186,9 @@ __device__ __forceinline__ void DrainCopies(Sync& S) {
 }
 
 // At the end of a CTA: the last one leaves the ticket and the counters at zero.
+// The arrivals of split tiles are back at zero by themselves (the last arrival
+// resets its counter) unless a wait ran out: a CTA that gave up never arrives, and
+// a count left behind would make a later launch sum partials that are not there.
 __device__ __forceinline__ void LeaveFlow(const FlowWork& w, int* lastCta) {
     if (threadIdx.x == 0) {
         __threadfence();
@@ -195,6 +198,8 @@ __device__ __forceinline__ void LeaveFlow(const FlowWork& w, int* lastCta) {
     __syncthreads();
     if (*lastCta) {
         for (int i = threadIdx.x; i < w.numDone; i += blockDim.x) w.done[i] = 0;
+        if (*reinterpret_cast<volatile int*>(w.status) & 2)
+            for (int i = threadIdx.x; i < w.numCounters; i += blockDim.x) w.counters[i] = 0;
         if (threadIdx.x < 2) w.ctrl[threadIdx.x] = 0;
     }
 }

@@ -1,6 +1,8 @@
-// One front, one row tile whose K range is split in two.  The second half waits
-// for a front that nothing finishes: the kernel gives up within its limit, reports
-// it in the status word and leaves its ticket and the fronts' counters at zero.
+// One front, one row tile whose K range is split in two.  First the second half
+// waits for a front that nothing finishes: the kernel gives up within its limit,
+// reports it in the status word and leaves every counter at zero.  Then the same
+// buffers solve the tile.
+#include <cmath>
 #include <complex>
 #include <cstdio>
 #include <cstring>
@@ -34,7 +36,7 @@ static int Run(int k, bool tc) {
     constexpr int s = FlowRows<R>(), half = s / 2, kCounters = 3, kDone = 4, kFlag = 3;
     const int cols = tc ? (k > 16 ? 32 : 16) : FlowCols(k);
     // G = [inv(L11)], lower triangular, and the panel's right-hand sides
-    std::vector<C> G((size_t)s * s), rhs((size_t)s * k);
+    std::vector<C> G((size_t)s * s), rhs((size_t)s * k), got((size_t)s * k);
     unsigned seed = 12345;
     auto next = [&] { seed = seed * 1664525u + 1013904223u; return (R)((int)(seed >> 8) % 2001 - 1000) / 1000; };
     for (int j = 0; j < s; ++j)
@@ -75,6 +77,7 @@ static int Run(int k, bool tc) {
     w.done = w.ctrl + 2;
     w.status = Device<int>(1);
     w.numDone = kDone;
+    w.numCounters = kCounters;
     PanelIO io;
     std::memset(&io, 0, sizeof(io));
     const FlowFront<R>* dFront = Device<FlowFront<R>>(1, &front);
@@ -88,17 +91,46 @@ static int Run(int k, bool tc) {
         LaunchFlow<R>(dFront, dTile, 2, k, nullptr, io, w, 0);
     };
     auto atRest = [&](int wantStatus) {
-        int ctrl[2 + kDone], status;
+        int counters[kCounters], ctrl[2 + kDone], status;
+        cudaMemcpy(counters, w.counters, sizeof(counters), cudaMemcpyDeviceToHost);
         cudaMemcpy(ctrl, w.ctrl, sizeof(ctrl), cudaMemcpyDeviceToHost);
         cudaMemcpy(&status, w.status, sizeof(status), cudaMemcpyDeviceToHost);
         bool ok = status == wantStatus;
+        for (int v : counters) ok = ok && v == 0;
         for (int v : ctrl) ok = ok && v == 0;
-        if (!ok) std::printf("status %d, ticket %d, done %d\n", status, ctrl[0], ctrl[2]);
+        if (!ok) std::printf("status %d, split counter %d, ticket %d, done %d\n", status, counters[0], ctrl[0], ctrl[2]);
         return ok;
     };
     launch();
     CHECK(cudaDeviceSynchronize());
     if (!atRest(2)) return 1;
+
+    tile[1].dep0 = -1;
+    CHECK(cudaMemcpy(dTile, tile, sizeof(tile), cudaMemcpyHostToDevice));
+    CHECK(cudaMemset(w.status, 0, sizeof(int)));
+    launch();
+    CHECK(cudaDeviceSynchronize());
+    if (!atRest(0)) return 1;
+    CHECK(cudaMemcpy(got.data(), w.w, got.size() * sizeof(C), cudaMemcpyDeviceToHost));
+    // s products per sum, each rounded (and added) to at most s units of the
+    // last place of the terms' sum of magnitudes
+    const double tol = (sizeof(R) == 4 ? 1.2e-7 : 2.3e-16) * s;
+    for (int i = 0; i < s; ++i)
+        for (int c = 0; c < k; ++c) {
+            std::complex<double> sum = 0;
+            double mag = 0;
+            for (int j = 0; j <= i; ++j) {
+                const std::complex<double> p = std::complex<double>(G[i + (size_t)j * s]) *
+                                               std::complex<double>(rhs[(size_t)j * k + c]);
+                sum += p;
+                mag += std::abs(p);
+            }
+            const double err = std::abs(std::complex<double>(got[(size_t)i * k + c]) - sum / 4.0);
+            if (!(err <= tol * mag)) {
+                std::printf("row %d column %d: off by %g of %g\n", i, c, err, mag);
+                return 1;
+            }
+        }
     return 0;
 }
 

@@ -1,8 +1,10 @@
 """A panel solve whose wait runs out.
 
 The kernels that walk the elimination tree bound every wait.  When one runs out
-(here on a counter that nothing sets) all roles of the CTA leave, the copies of
-factors still in flight land first, and the status word reports it.
+(here on a counter that nothing sets) they report it in the status word, and
+what later launches start from, the ticket, the fronts' counters and the
+arrivals of split tiles, is at zero again: a count left behind made the next
+solve on the same plan sum partial tiles that were not written yet.
 """
 import os
 import shutil
@@ -31,6 +33,6 @@ def test_driver_compiles(driver):
 
 
 @pytest.mark.gpu
-def test_gives_up_and_reports(driver):
+def test_counters_are_at_zero_after_a_wait_ran_out(driver):
     r = subprocess.run([driver], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, r.stdout + r.stderr
