@@ -189,8 +189,8 @@ public:
     // Frees the solve plans (and the sweep graphs that use them) of every
     // block width but k.
     void DropPlansExcept(int k);
-    // Device status word: bit 1 zero/non-finite pivot, bit 2 a tensor-core
-    // pipeline wait timed out.  Synchronizes the stream.
+    // Device status word: bit 1 zero/non-finite pivot, bit 2 a bounded wait of
+    // a kernel ran out.  Synchronizes the stream.
     int ReadStatus() {
         int st = 0;
         CUDA_CHECK(cudaMemcpyAsync(&st, status_.p, sizeof(int), cudaMemcpyDeviceToHost, h_.stream_));
@@ -1372,7 +1372,7 @@ void Helmholtz::Precondition(z64* B, int k, bool useGraph) {
 void Helmholtz::CheckSweepStatus() {
     const int st = f64_ ? f64_->ReadStatus() : (f32_ ? f32_->ReadStatus() : 0);
     if (st & 1) throw PspError(kRuntimeError, "zero or non-finite pivot in a recomputed panel factorization");
-    if (st & 2) throw PspError(kRuntimeError, "a tensor-core pipeline wait timed out in the sweep");
+    if (st & 2) throw PspError(kRuntimeError, "a wait ran out in a panel solve of the sweep or in a recomputed panel's factorization");
 }
 
 void Helmholtz::PreconditionDevice(z64* B, int k) {
@@ -1396,6 +1396,7 @@ void Helmholtz::SolvePanelDevice(z64* B, int k, int panel) {
         else f32_->SolvePanel(B + r0, k, kb, panel, 0, 0);
     }
     CUDA_CHECK(cudaStreamSynchronize(stream_));
+    CheckSweepStatus();
 }
 
 void Helmholtz::SetPanelRange(int p0, int p1) {
