@@ -218,9 +218,7 @@ __device__ void LoaderRole(int k, unsigned char* smem, Sync<R>& S, const PanelIO
                     at[i] = t.bwd && row < rows && kk >= f.s && kk < t.ke ? __ldg(f.lower + kk - f.s) : f.ndOff + kk;
                 }
                 if (!waited) {
-                    const int dep = lane == 0 ? t.dep0 : lane == 1 ? t.dep1 : -1;
-                    const bool ok = dep < 0 || WaitCount(w.done + dep, lane ? t.need1 : t.need0, S, w.status);
-                    if (!__all_sync(~0u, ok)) return;
+                    if (!TileReady(t, true, S, w)) return;
                     waited = true;
                 }
                 Unit<R, V> v[kBatch], p0[kBatch], p1[kBatch];

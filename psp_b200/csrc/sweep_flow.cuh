@@ -60,6 +60,20 @@ __device__ __forceinline__ bool WaitCount(const int* p, int target, Sync& S, int
     return false;
 }
 
+// Whether the fronts that a tile reads are finished, tested once (`wait` false) or
+// waited for (bounded); by a whole warp.  Two lanes acquire the counters.  A vote
+// passes their answer on but orders no memory; the warp barrier after it does, so
+// that every lane's loads see what those fronts' tiles wrote.
+template <typename Sync>
+__device__ __forceinline__ bool TileReady(const FlowTile& t, bool wait, Sync& S, const FlowWork& w) {
+    const int lane = threadIdx.x & 31;
+    const int dep = lane == 0 ? t.dep0 : lane == 1 ? t.dep1 : -1, need = lane ? t.need1 : t.need0;
+    const bool ok = dep < 0 || (wait ? WaitCount(w.done + dep, need, S, w.status) : LoadAcquire(w.done + dep) >= need);
+    const bool all = __all_sync(~0u, ok);
+    __syncwarp();
+    return all;
+}
+
 // Global data written by other CTAs of this launch: through L2.
 __device__ __forceinline__ c32 LoadCg(const c32* p) {
     const float2 v = __ldcg(reinterpret_cast<const float2*>(p));

@@ -263,11 +263,10 @@ __device__ void LoaderRole(int k, unsigned char* smem, Sync& S, const FlowWork& 
             }
             if (!ready) {
                 const FlowTile& t = S.queue[q % kQueue].t;
-                const int dep = lane == 0 ? t.dep0 : lane == 1 ? t.dep1 : -1, need = lane ? t.need1 : t.need0;
-                ready = __all_sync(~0u, dep < 0 || LoadAcquire(w.done + dep) >= need);
+                ready = TileReady(t, false, S, w);
                 if (!ready) {
                     if (pending > 0) break;  // split what is here first
-                    ready = __all_sync(~0u, dep < 0 || WaitCount(w.done + dep, need, S, w.status));
+                    ready = TileReady(t, true, S, w);
                     if (!ready) { done = true; break; }
                 }
             }
@@ -622,9 +621,7 @@ __device__ void EpilogueRole(int k, Sync& S, z64* B, const PanelIO& io, const Fl
                 o.dst = f.Pp + (int64_t)__ldg(f.rel + r - s) * k;
             }
             if (t.carry) {  // into the sum while the tile's stages run
-                const int dep = lane == 0 ? t.dep0 : lane == 1 ? t.dep1 : -1;
-                ok = dep < 0 || WaitCount(w.done + dep, lane ? t.need1 : t.need0, S, w.status);
-                ok = __all_sync(~0u, ok);
+                ok = TileReady(t, true, S, w);
                 if (ok) {
                     const bool in = r >= s && r < s + f.u;
                     const c32* c0 = in && f.P0 ? f.P0 + (int64_t)r * k + col0 : nullptr;
