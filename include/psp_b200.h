@@ -127,8 +127,9 @@ int psp_cu_precondition_device(psp_cu_handle* h, double* d_B, int k);
  * while they call -- code running inside its own CUDA stream capture, where an
  * allocation breaks the capture, and services that reserve all device memory
  * up front.  psp_cu_multiply_device keeps its temporary (nx*ny*nz*k entries, at
- * most 1 GiB) with the handle until psp_cu_finalize and allocates when a call
- * needs more than is kept; this variant uses a 16 MiB file-scope device array instead, so
+ * most 1 GiB) with the handle until psp_cu_finalize, or until another call of the
+ * handle is short of memory, and allocates when a call needs more than is kept;
+ * this variant uses a 16 MiB file-scope device array instead, so
  * nx*ny*nz*k must not exceed 1048576 (PSP_CU_LOGIC_ERROR otherwise).  The
  * first call on a device looks up that array's device address; make it before
  * any stream capture.  All calls share the array: calls that overlap on the

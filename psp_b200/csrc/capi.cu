@@ -68,7 +68,7 @@ void OnDeviceCopy(psp_cu_handle* h, double* B, int k, F&& fn) {
     Helmholtz* s = h->solver;
     CUDA_CHECK(cudaSetDevice(s->device()));
     const size_t bytes = (size_t)s->NumUnknowns() * k * 2 * sizeof(double);
-    void* d = h->io.Device(bytes);
+    void* d = s->WithRoom([&] { return h->io.Device(bytes); });
     h->io.ToDevice(d, B, bytes, s->stream());
     fn(static_cast<psp_b200::z64*>(d));
     h->io.ToHost(B, d, bytes, s->stream());
@@ -119,7 +119,7 @@ int psp_cu_initialize(psp_cu_handle* h, const double* velocity, int panel_scheme
         if (!velocity) return h->solver->Initialize(nullptr, false, panel_scheme, precision);
         CUDA_CHECK(cudaSetDevice(h->solver->device()));
         const size_t bytes = (size_t)h->solver->NumUnknowns() * sizeof(double);
-        void* d = h->io.Device(bytes);
+        void* d = h->solver->WithRoom([&] { return h->io.Device(bytes); });
         h->io.ToDevice(d, velocity, bytes, h->solver->stream());
         h->solver->Initialize(static_cast<const double*>(d), true, panel_scheme, precision);
     });

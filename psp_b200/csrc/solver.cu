@@ -285,6 +285,7 @@ private:
     };
     std::vector<std::unique_ptr<SolvePlan>> plans_;
     SolvePlan& Plan(int k);
+    void BuildPlan(int k);
     bool tc_ = false;  // tensor-core sweep kernel (complex single only)
     bool factorTc_ = false;  // tensor-core factorization GEMMs (complex single only)
     // Ops of at least this many rows and K columns take tensor-core tiles.
@@ -495,9 +496,7 @@ void FactorStore<R>::Factor() {
             if (resident_[p]) res.push_back(p);
         // groups of resident panels whose transients fit in 80% of the free
         // memory (the scratch counts as free: it is reused)
-        size_t freeB = 0, totalB = 0;
-        CUDA_CHECK(cudaMemGetInfo(&freeB, &totalB));
-        const int64_t budget = (int64_t)(0.8 * ((double)freeB + (double)h_.ScratchBytes()));
+        const int64_t budget = (int64_t)(0.8 * h_.RoomBytes());
         int groupSize = std::max<int>(1, (int)res.size());
         auto slice = [&](size_t i0, int n) {
             return std::vector<int>(res.begin() + i0, res.begin() + std::min(res.size(), i0 + n));
@@ -509,6 +508,7 @@ void FactorStore<R>::Factor() {
         };
         while (groupSize > 1 && maxTransient(groupSize) > budget) groupSize = (groupSize + 1) / 2;
         const int64_t need = res.empty() ? 0 : maxTransient(groupSize);
+        h_.MakeRoom(need / 0.8);
         unsigned char* arena = static_cast<unsigned char*>(h_.Scratch(need));
         for (size_t i0 = 0; i0 < res.size(); i0 += groupSize)
             program_.push_back(FactorGroup(slice(i0, groupSize), arena, need));
@@ -811,6 +811,12 @@ template <typename R>
 typename FactorStore<R>::SolvePlan& FactorStore<R>::Plan(int k) {
     for (auto& pl : plans_)
         if (pl->k == k) return *pl;
+    h_.WithRoom([&] { BuildPlan(k); });
+    return *plans_.back();
+}
+
+template <typename R>
+void FactorStore<R>::BuildPlan(int k) {
     std::unique_ptr<SolvePlan> plan(new SolvePlan);
     SolvePlan& P = *plan;
     P.k = k;
@@ -1013,7 +1019,6 @@ typename FactorStore<R>::SolvePlan& FactorStore<R>::Plan(int k) {
     CUDA_CHECK(cudaMemcpyAsync(P.maps.p, P.mapsHost.data(), P.maps.bytes, cudaMemcpyHostToDevice, h_.stream_));
     CUDA_CHECK(cudaStreamSynchronize(h_.stream_));
     plans_.push_back(std::move(plan));
-    return P;
 }
 
 template <typename R>
@@ -1308,16 +1313,35 @@ void Helmholtz::Finalize() {
     initialized_ = false;
 }
 
-void Helmholtz::ReleaseApplyRing() {
+bool Helmholtz::ReleaseApplyRing() {
     std::lock_guard<std::mutex> lock(applyMutex_);
-    if (applyRing_.p) cudaStreamSynchronize(stream_);
+    if (!applyRing_.p) return false;
+    cudaStreamSynchronize(stream_);
     applyRing_.Release();
+    return true;
+}
+
+double Helmholtz::RoomBytes() {
+    std::lock_guard<std::mutex> lock(applyMutex_);
+    size_t freeB = 0, totalB = 0;
+    CUDA_CHECK(cudaMemGetInfo(&freeB, &totalB));
+    return (double)freeB + (double)pool_.bytes + (double)applyRing_.bytes;
+}
+
+void Helmholtz::MakeRoom(double bytes) {
+    {
+        std::lock_guard<std::mutex> lock(applyMutex_);
+        if (!applyRing_.p) return;
+    }
+    size_t freeB = 0, totalB = 0;
+    CUDA_CHECK(cudaMemGetInfo(&freeB, &totalB));
+    if (bytes > (double)freeB + (double)pool_.bytes) ReleaseApplyRing();
 }
 
 void* Helmholtz::Scratch(size_t bytes) {
     if (bytes > pool_.bytes) {
         pool_.Release();
-        pool_.Allocate(bytes);
+        WithRoom([&] { pool_.Allocate(bytes); });
     }
     return pool_.p;
 }
@@ -1447,8 +1471,8 @@ void Helmholtz::MultiplySlab(const z64* X, z64* Y, const z64* Bv, int k, int zFi
 }
 
 // Memory that MultiplyDevice keeps between calls (an allocation takes 1 to 30 ms,
-// the launches of a 400 MB grid 0.3 ms); more than that, where a single plane
-// is larger than a third of it, is freed again.
+// the launches of a 400 MB grid 0.3 ms) while the factors are there too; more than
+// that, where a single plane is larger than a third of it, is freed again.
 constexpr size_t kKeptApplyRing = size_t(1) << 30;
 
 void Helmholtz::MultiplyDevice(z64* B, int k) {
@@ -1462,7 +1486,7 @@ void Helmholtz::MultiplyDevice(z64* B, int k) {
             applyRing_.Allocate(need);
         }
         LaunchHelmholtzInPlace(B, applyRing_.p, dVel_.as<double>(), sp_, k, stream_);
-        if (applyRing_.bytes > kKeptApplyRing) {
+        if (applyRing_.bytes > kKeptApplyRing || !initialized_) {
             CUDA_CHECK(cudaStreamSynchronize(stream_));
             applyRing_.Release();
         }
@@ -1524,17 +1548,21 @@ bool AnyNaN(const std::vector<double>& v) {
 }  // namespace
 
 double Helmholtz::GmresBytesPerRhs(int m) const {
-    // V (m vectors), x, x0, w, b and a block's copy of its columns, the
-    // solve plan's work vectors and the sweep autotuner's scratch
+    // V (m vectors), x, x0, w, b, a block's copy of its columns and one vector's
+    // worth for the reductions, split tiles and task lists, and the solve
+    // plan's work vectors
     double plan = 0;
     if (f64_) plan = f64_->PlanBytesPerRhs();
     if (f32_) plan = f32_->PlanBytesPerRhs();
     return (double)NumUnknowns() * sizeof(z64) * (m + 6) + plan;
 }
 
+// Of the memory left beside this margin, the part that the workspace may take.
+constexpr double kGmresMargin = 0.5e9, kGmresShare = 0.95;
+
 int ChooseBlockWidth(int k, double availBytes, double perRhsBytes, int cap) {
     if (k < 1 || perRhsBytes <= 0) throw PspError(kLogicError, "need k >= 1 and a positive workspace size");
-    const double fitD = std::floor(0.95 * availBytes / perRhsBytes);
+    const double fitD = std::floor(kGmresShare * availBytes / perRhsBytes);
     if (fitD < 1)
         throw PspError(kOutOfMemory, "the GMRES workspace of one right-hand side (" +
                                          std::to_string(perRhsBytes / 1e9) + " GB) does not fit in the " +
@@ -1554,11 +1582,9 @@ int ChooseBlockWidth(int k, double availBytes, double perRhsBytes, int cap) {
 
 int Helmholtz::GmresBlockWidth(int k, int m) {
     const long long cap = EnvInt("PSP_B200_MAX_RHS_BLOCK", 0);
-    size_t freeB = 0, totalB = 0;
-    CUDA_CHECK(cudaMemGetInfo(&freeB, &totalB));
     // the scratch is reused for the workspace; the plan of the current width
     // (when built) is already counted as used memory
-    const double avail = (double)freeB + (double)pool_.bytes - 0.5e9;
+    const double avail = RoomBytes() - kGmresMargin;
     return ChooseBlockWidth(k, avail, GmresBytesPerRhs(m), cap > 0 ? (int)std::min<long long>(cap, k) : 0);
 }
 
@@ -1568,6 +1594,7 @@ void Helmholtz::SolveDevice(z64* B, int k, int m, double relTol, SolveStats* sta
     if (m < 1) throw PspError(kLogicError, "GMRES restart length must be positive");
     CUDA_CHECK(cudaSetDevice(device_));
     const int kb = GmresBlockWidth(k, m);
+    MakeRoom(kb * GmresBytesPerRhs(m) / kGmresShare + kGmresMargin);
     if (kb >= k) {
         EnsureWorkspace(k, m, false);
         SolveBlock(B, k, m, relTol, stats);

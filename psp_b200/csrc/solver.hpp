@@ -166,6 +166,23 @@ public:
     void* Scratch(size_t bytes);
     size_t ScratchBytes() const { return pool_.bytes; }
 
+    // The planes that MultiplyDevice keeps are no one's loss: what they take
+    // counts as available (RoomBytes: free memory, the scratch and these planes),
+    // MakeRoom gives them back unless `bytes` of that are there without them, and
+    // an allocation that fails is tried again without them (WithRoom).
+    double RoomBytes();
+    void MakeRoom(double bytes);
+    template <typename F>
+    auto WithRoom(F&& allocate) -> decltype(allocate()) {
+        try {
+            return allocate();
+        } catch (const PspError& e) {
+            if (e.code != kOutOfMemory || !ReleaseApplyRing()) throw;
+            cudaGetLastError();  // the failure is dealt with
+        }
+        return allocate();
+    }
+
     // Device tables shared with the factor stores.
     StencilParams sp_{};
     AssemblyParams ap_{};
@@ -212,7 +229,7 @@ private:
     // them and the stream's order)
     DeviceBuffer applyRing_;
     std::mutex applyMutex_;
-    void ReleaseApplyRing();
+    bool ReleaseApplyRing();  // false when there were none
     // GMRES workspace, carved from pool_ by EnsureWorkspace
     z64 *wsX_ = nullptr, *wsX0_ = nullptr, *wsW_ = nullptr, *wsB_ = nullptr, *wsV_ = nullptr;
     z64 *wsCols_ = nullptr, *wsY_ = nullptr;
