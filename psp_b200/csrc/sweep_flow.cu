@@ -134,9 +134,10 @@ __device__ void ProducerRole(const FlowFront<R>* __restrict__ fr, const FlowTile
     TileSource<R> src;
     src.Start(fr, tiles, n, w.ctrl, false);
     int g = 0;
+    bool ok = true;
     for (int q = 0;; ++q) {
         const int qs = q % kQueue;
-        if (q >= kQueue && !WaitWarp(&S.tileEmpty[qs], ((q / kQueue) - 1) & 1, S, w.status)) return;
+        if (q >= kQueue && !WaitWarp(&S.tileEmpty[qs], ((q / kQueue) - 1) & 1, S, w.status)) break;
         if (lane < kCtxWords) reinterpret_cast<int4*>(&S.queue[qs])[lane] = src.ctx;
         __syncwarp();
         if (lane == 0) umma::MbarArrive(&S.tileFull[qs]);
@@ -146,7 +147,8 @@ __device__ void ProducerRole(const FlowFront<R>* __restrict__ fr, const FlowTile
         const int nst = t.nst;
         for (int st = 0; st < nst; ++st, ++g) {
             const int slot = g % C::kSlots;
-            if (g >= C::kSlots && !WaitWarp(&S.empty[slot], ((g / C::kSlots) - 1) & 1, S, w.status)) return;
+            ok = g < C::kSlots || WaitWarp(&S.empty[slot], ((g / C::kSlots) - 1) & 1, S, w.status);
+            if (!ok) break;
             if (lane == 0) {
                 unsigned char* dst = smem + slot * kGBytes;
                 const int kBase = t.k0 + st * kStageK;
@@ -159,12 +161,13 @@ __device__ void ProducerRole(const FlowFront<R>* __restrict__ fr, const FlowTile
                     TmaLoadStream(dst, map, 2 * kBase, t.row0, &S.tma[slot], policy);
                     TmaLoadStream(dst + kGBytes / 2, map, 2 * kBase + kStageK, t.row0, &S.tma[slot], policy);
                 }
-                S.issued = g + 1;
             }
             __syncwarp();
         }
+        if (!ok) break;
         src.Take();
     }
+    if (lane == 0) S.issued = g;  // read after all roles have returned
 }
 
 // ------------------------------------------------------------------ loaders
