@@ -105,6 +105,8 @@ constexpr int kNB = 32;  // column block of the frontal LDL^T
 // even, so that every column starts on a 16-byte boundary for bulk copies
 // (the padding row is zero).
 __host__ __device__ inline int GLeadingDim(int s, int u) { return (s + u + 1) & ~1; }
+// Nonzeros of a front's G.
+inline double GNonzeros(double s, double u) { return (s + u) * s - s * (s - 1) / 2; }
 
 // One front of one panel during the factorization (cliq::LDL replacement).
 template <typename R>
@@ -221,8 +223,17 @@ struct FlowWork {
     int numDone, numCounters;
 };
 
-// Columns of a tile for k right-hand sides: the power of two that holds them, at most kFlowMaxCols.
-int FlowCols(int k);
+// Columns of a tile of the CUDA-core kernel for k right-hand sides: the power of
+// two that holds them up to 16, else 16, or 32 (kFlowMaxCols) where that is the
+// faster one.  `stages`: stages of one panel solve per CTA that runs at once
+// and column tile.  A tile of 32 columns takes twice as long per stage, and half of
+// it is idle when the 16-column tiles are odd in number; it reads G half as often,
+// which pays where wide levels, not the chain of levels, are most of the time.
+// Sweeps with 32 instead of 16 columns, time against stages * ceil(k / 16): FP64
+// k = 17 to 32: +36 % at 32, +8 % at 270, +1 % at 640, -1 % at 750, -5 % at 1780;
+// k = 64: +33 % at 64, +3 % at 540, -1 % at 740, -6 % at 3560; k = 33 to 48: +22 % and
+// more everywhere; complex single crosses between 500 and 900.
+int FlowCols(int k, double stages);
 template <typename R>
 int FlowCarryChunks(int cols);
 // CTAs that run at once.
@@ -235,7 +246,7 @@ void EncodeFlowMaps(const cpx<R>* G, int s, int u, int ldg, void* out);
 template <typename R>
 void LaunchFlowGather(const z64* B, cpx<R>* rnd, int own, int k, const PanelIO& io, cudaStream_t st);
 template <typename R>
-void LaunchFlow(const FlowFront<R>* fr, const FlowTile* tiles, int n, int k, z64* B, const PanelIO& io,
+void LaunchFlow(const FlowFront<R>* fr, const FlowTile* tiles, int n, int k, int cols, z64* B, const PanelIO& io,
                 const FlowWork& w, cudaStream_t st);
 // The same tile list on the tensor cores (sweep_flow_tc.cu; complex single,
 // `cols` 16 or 32 right-hand sides per tile).

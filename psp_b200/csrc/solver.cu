@@ -825,9 +825,8 @@ void FactorStore<R>::BuildPlan(int k) {
     const int np = g.numPanels, nd = (int)depthNodes_.size();
     constexpr int TR = FlowRows<R>();
     P.tc = tc_ && k >= kFlowTcMinCols;
-    const int nc = P.cols = P.tc ? (k > 16 ? 32 : 16) : FlowCols(k);
-    const int carryChunks = P.tc ? 1 : FlowCarryChunks<R>(nc);
     const int running = P.tc ? FlowTcSlots() : FlowSlots();  // CTAs that run at once
+    double mostNz = 0;  // nonzeros of G of the largest panel class
     // per front two planes of s + u rows, one per child
     int maxSub = 0;
     int64_t maxRows = 0;
@@ -842,7 +841,12 @@ void FactorStore<R>::BuildPlan(int k) {
             if (tree.nodes[t].numChildren > 0) rows += 2 * (int64_t)(an_.cls[c].size[t] + an_.cls[c].usize[t]);
         }
         maxRows = std::max(maxRows, rows);
+        double nz = 0;
+        for (int t = 0; t < nn_; ++t) nz += GNonzeros(an_.cls[c].size[t], an_.cls[c].usize[t]);
+        mostNz = std::max(mostNz, nz);
     }
+    const int nc = P.cols = P.tc ? (k > 16 ? 32 : 16) : FlowCols(k, mostNz / ((double)TR * kFlowStageK * running));
+    const int carryChunks = P.tc ? 1 : FlowCarryChunks<R>(nc);
     P.rnd.Allocate((size_t)maxSub * k * sizeof(cpx<R>));
     P.W.Allocate((size_t)maxSub * k * sizeof(cpx<R>));
     P.X.Allocate((size_t)maxSub * k * sizeof(cpx<R>));
@@ -1005,7 +1009,7 @@ void FactorStore<R>::BuildPlan(int k) {
         P.tiles[c] = P.arena.Push(list);
         for (int t = 0; t < nn_; ++t) {
             const double s = cs.size[t], u = cs.usize[t];
-            const double nz = (s + u) * s - s * (s - 1) / 2;  // nonzeros of G
+            const double nz = GNonzeros(s, u);
             P.flops[c] += 2 * 8.0 * nz * k;
             P.bytes[c] += sizeof(cpx<R>) * (2 * nz + (s + 2 * (s + u) + 2 * (s + u) + 2 * s) * k);
         }
@@ -1075,7 +1079,7 @@ void FactorStore<R>::SolvePanel(z64* B, int ldk, int k, int p, int inMode, int o
             return;
         }
     }
-    LaunchFlow<R>(fr, tiles, P.numTiles[c], k, B, io, w, st);
+    LaunchFlow<R>(fr, tiles, P.numTiles[c], k, P.cols, B, io, w, st);
 }
 
 template <typename R>
@@ -1160,7 +1164,7 @@ double FactorStore<R>::SweepFlops(int k) const {
         double pf = 0;
         for (size_t t = 0; t < cs.size.size(); ++t) {
             const double s = cs.size[t], u = cs.usize[t];
-            pf += 8.0 * k * 2 * ((s + u) * s - s * (s - 1) / 2);
+            pf += 8.0 * k * 2 * GNonzeros(s, u);
         }
         f += (p == g.numPanels - 1 ? 1 : 2) * pf;
     }
@@ -1176,7 +1180,7 @@ double FactorStore<R>::SweepBytes(int k) const {
         double pb = 0;
         for (size_t t = 0; t < cs.size.size(); ++t) {
             const double s = cs.size[t], u = cs.usize[t];
-            pb += 2.0 * sizeof(cpx<R>) * ((s + u) * s - s * (s - 1) / 2);
+            pb += 2.0 * sizeof(cpx<R>) * GNonzeros(s, u);
         }
         pb += 2.0 * 16.0 * k * g.Depth(p) * an_.disc.nx * an_.disc.ny;  // natural-order RHS in and out
         b += (p == g.numPanels - 1 ? 1 : 2) * pb;

@@ -768,10 +768,13 @@ void PrepareNc() {
 
 }  // namespace
 
-int FlowCols(int k) {
+int FlowCols(int k, double stages) {
     int nc = 1;
-    while (nc < k && nc < kFlowMaxCols) nc *= 2;
-    return nc;
+    while (nc < k && nc < kFlowMaxCols / 2) nc *= 2;
+    if (k <= nc) return nc;
+    constexpr double kWideStages = 700;
+    const int narrow = (int)CeilDiv(k, nc);
+    return narrow % 2 == 0 && narrow * stages >= kWideStages ? kFlowMaxCols : nc;
 }
 
 template <typename R>
@@ -830,10 +833,10 @@ void LaunchFlowGather(const z64* B, cpx<R>* rnd, int own, int k, const PanelIO& 
 }
 
 template <typename R>
-void LaunchFlow(const FlowFront<R>* fr, const FlowTile* tiles, int n, int k, z64* B, const PanelIO& io, const FlowWork& w,
-                cudaStream_t st) {
+void LaunchFlow(const FlowFront<R>* fr, const FlowTile* tiles, int n, int k, int cols, z64* B, const PanelIO& io,
+                const FlowWork& w, cudaStream_t st) {
     if (n <= 0) return;
-    switch (FlowCols(k)) {
+    switch (cols) {
         case 1: LaunchNc<R, 1>(fr, tiles, n, k, B, io, w, st); break;
         case 2: LaunchNc<R, 2>(fr, tiles, n, k, B, io, w, st); break;
         case 4: LaunchNc<R, 4>(fr, tiles, n, k, B, io, w, st); break;
@@ -848,8 +851,8 @@ void LaunchFlow(const FlowFront<R>* fr, const FlowTile* tiles, int n, int k, z64
     template void PrepareFlowKernels<R>();                                                                            \
     template void EncodeFlowMaps<R>(const cpx<R>*, int, int, int, void*);                                             \
     template void LaunchFlowGather<R>(const z64*, cpx<R>*, int, int, const PanelIO&, cudaStream_t);                   \
-    template void LaunchFlow<R>(const FlowFront<R>*, const FlowTile*, int, int, z64*, const PanelIO&, const FlowWork&, \
-                                cudaStream_t);
+    template void LaunchFlow<R>(const FlowFront<R>*, const FlowTile*, int, int, int, z64*, const PanelIO&,            \
+                                const FlowWork&, cudaStream_t);
 
 PSP_FLOW_INSTANTIATE(double)
 PSP_FLOW_INSTANTIATE(float)
