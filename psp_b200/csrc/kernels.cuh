@@ -199,16 +199,15 @@ struct alignas(16) FlowFront {
 
 // One tile: rows row0 .. of front `front`, columns col0 .., K range [k0, ke)
 // in nst stages (and `carry` chunks of the children's updates of its update
-// rows); split `split` of `nsplit`.  It may start once done[dep0] >= need0 and
-// done[dep1] >= need1 (-1: no such dependency) and adds one to done[signal]
-// when its output is written.
+// rows); split `split` of `nsplit`.  It may start once done[dep] >= need0 and
+// done[dep + 1] >= need1 (dep even; -1: it waits for nothing) and adds one to
+// done[signal] when its output is written.
 struct alignas(16) FlowTile {
     int front, row0, col0, k0;
-    int ke, nst, dep0, need0;
-    int dep1, need1, signal, slot;
-    int counter;
+    int ke, nst, dep, need0;
+    int need1, signal, slot, counter;
     short split, nsplit, carry, bwd;
-    int pad;
+    int pad[2];
 };
 
 struct FlowWork {
@@ -217,7 +216,7 @@ struct FlowWork {
     void* x;         // [nSub][k] solution
     void* partials;  // split-K partial tiles
     int* counters;   // arrivals of split tiles (zero between launches)
-    int* done;       // finished tiles per front, forward then backward (zero between launches)
+    int* done;       // finished tiles per front and direction, in pairs (8-byte aligned; zero between launches)
     int* ctrl;       // ticket, finished CTAs (zero between launches)
     int* status;     // bit 2: a wait timed out
     int numDone, numCounters;

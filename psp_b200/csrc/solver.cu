@@ -902,6 +902,13 @@ void FactorStore<R>::BuildPlan(int k) {
     };
     const long long fixedEnv = P.tc ? EnvInt("PSP_B200_SWEEP_TC_CHUNK", 0) : 0;
     const long long maxEnv = P.tc ? EnvInt("PSP_B200_SWEEP_TC_MAX_CHUNK", 0) : 0;
+    // Counters of finished tiles, in pairs that a tile reads at once: the
+    // forward ones of a front's children, the root's, then each front's backward one.
+    auto forwardCount = [&](int t) {
+        const int up = tree.nodes[t].parent;
+        return up < 0 ? 2 * nn_ : 2 * up + (tree.nodes[up].child[1] == t ? 1 : 0);
+    };
+    auto backwardCount = [&](int t) { return 2 * (nn_ + 1 + t); };
     int64_t maxSlots = 1, maxCounters = 1;
     for (int c = 0; c < 3; ++c) {
         if (!an_.classUsed[c]) continue;
@@ -967,21 +974,21 @@ void FactorStore<R>::BuildPlan(int k) {
                         FlowTile tl;
                         std::memset(&tl, 0, sizeof(tl));
                         tl.front = t; tl.row0 = row0; tl.col0 = col0;
-                        tl.dep0 = tl.dep1 = -1;
+                        tl.dep = -1;
                         tl.bwd = !fwd;
-                        tl.signal = fwd ? t : nn_ + t;
+                        tl.signal = fwd ? forwardCount(t) : backwardCount(t);
                         if (fwd) {
                             for (int slot = 0; slot < node.numChildren; ++slot) {
                                 const int ch = node.child[slot];
                                 if (cs.size[ch] == 0) continue;
-                                (slot ? tl.dep1 : tl.dep0) = ch;
+                                tl.dep = 2 * t;
                                 (slot ? tl.need1 : tl.need0) = outputs(ch, true);
                             }
                         } else if (node.parent >= 0) {
-                            tl.dep0 = nn_ + node.parent;
+                            tl.dep = backwardCount(node.parent);
                             tl.need0 = outputs(node.parent, false);
                         } else {
-                            tl.dep0 = t;
+                            tl.dep = forwardCount(t);
                             tl.need0 = outputs(t, true);
                         }
                         const int parts = (int)CeilDiv(nst, per);
@@ -1016,7 +1023,7 @@ void FactorStore<R>::BuildPlan(int k) {
     }
     P.partials.Allocate((size_t)maxSlots * TR * nc * sizeof(cpx<R>));
     P.counters.Allocate((size_t)maxCounters * sizeof(int));
-    P.done.Allocate((2 * (size_t)nn_ + 2) * sizeof(int));
+    P.done.Allocate((4 * (size_t)nn_ + 4) * sizeof(int));
     CUDA_CHECK(cudaMemsetAsync(P.counters.p, 0, P.counters.bytes, h_.stream_));
     CUDA_CHECK(cudaMemsetAsync(P.done.p, 0, P.done.bytes, h_.stream_));
     P.arena.Upload(h_.stream_);
@@ -1055,7 +1062,7 @@ void FactorStore<R>::SolvePanel(z64* B, int ldk, int k, int p, int inMode, int o
     w.counters = P.counters.template as<int>();
     w.ctrl = P.done.template as<int>();
     w.done = w.ctrl + 2;
-    w.numDone = 2 * nn_;
+    w.numDone = (int)(P.done.bytes / sizeof(int)) - 2;
     w.numCounters = (int)(P.counters.bytes / sizeof(int));
     w.status = status_.template as<int>();
     {

@@ -33,7 +33,7 @@ static T* Device(size_t n, const T* src = nullptr) {
 template <typename R>
 static int Run(int k, int cols, bool tc) {
     typedef std::complex<R> C;
-    constexpr int s = FlowRows<R>(), half = s / 2, kCounters = 3, kDone = 4, kFlag = 3;
+    constexpr int s = FlowRows<R>(), half = s / 2, kCounters = 3, kDone = 4, kFlag = 2;
     // G = [inv(L11)], lower triangular, and the panel's right-hand sides
     std::vector<C> G((size_t)s * s), rhs((size_t)s * k), got((size_t)s * k);
     unsigned seed = 12345;
@@ -59,11 +59,11 @@ static int Run(int k, int cols, bool tc) {
         t.k0 = sp * half;
         t.ke = t.k0 + half;
         t.nst = half / kFlowStageK;
-        t.dep0 = t.dep1 = -1;
+        t.dep = -1;
         t.split = (short)sp;
         t.nsplit = 2;
     }
-    tile[1].dep0 = kFlag;  // nothing finishes this front
+    tile[1].dep = kFlag;  // nothing finishes this front
     tile[1].need0 = 1;
     FlowWork w;
     std::memset(&w, 0, sizeof(w));
@@ -104,7 +104,7 @@ static int Run(int k, int cols, bool tc) {
     CHECK(cudaDeviceSynchronize());
     if (!atRest(2)) return 1;
 
-    tile[1].dep0 = -1;
+    tile[1].dep = -1;
     CHECK(cudaMemcpy(dTile, tile, sizeof(tile), cudaMemcpyHostToDevice));
     CHECK(cudaMemset(w.status, 0, sizeof(int)));
     launch();
