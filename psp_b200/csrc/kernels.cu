@@ -43,9 +43,9 @@ __device__ __forceinline__ Terms StencilAt(const StencilParams& sp, int x, int y
 
 // ---------------------------------------------------------------- stencil apply
 
-// A block applies the operator to kApplyTX points of a row: one thread per
-// point for the coefficients (products and quotients of the stretch tables),
-// then one per column and point, all seven entries in flight.  Eight blocks per
+// A block applies the operator to up to kApplyTX points of a row (`px`, chosen by
+// ApplyPoints): one thread per point for the coefficients (products and quotients of
+// the stretch tables), then one per column and point, all seven entries in flight.  Eight blocks per
 // SM hide the first part behind the second.  Bound by memory: 140 x 140 x 80,
 // k = 32 (0.8 GB in, 0.8 GB out, b in every second launch): 0.45 ms with 64
 // points on 256 threads, most of them idle through the coefficients, now 0.42 ms
@@ -53,16 +53,16 @@ __device__ __forceinline__ Terms StencilAt(const StencilParams& sp, int x, int y
 // fewer warps in flight and take 0.44 and 0.69 ms.
 constexpr int kApplyTX = 128;
 
-// out(e, (A x) at entry e of the row piece); `base` is the piece's first point
-// in x's storage, `ready` runs before the first use of x.
+// out(e, (A x) at entry e of the row piece); `base` is the first of the piece's px
+// points in x's storage, `ready` runs before the first use of x.
 template <typename Ready, typename Out>
 __device__ __forceinline__ void ApplyRow(const z64* __restrict__ x, const double* __restrict__ vel,
-                                         const StencilParams& sp, int k, int x0, int yy, int zz, int64_t base,
+                                         const StencilParams& sp, int k, int px, int x0, int yy, int zz, int64_t base,
                                          const Ready& ready, const Out& out) {
     __shared__ z64 coef[kApplyTX][7];
     const int nx = sp.nx, ny = sp.ny, nz = sp.nz;
     const int64_t nxy = (int64_t)nx * ny;
-    const int npts = min(kApplyTX, nx - x0);
+    const int npts = min(px, nx - x0);
     const int v = nz - 1 - zz;
     if ((int)threadIdx.x < npts) {
         const int xx = x0 + threadIdx.x;
@@ -105,10 +105,10 @@ __device__ __forceinline__ void ApplyRow(const z64* __restrict__ x, const double
 __global__ void __launch_bounds__(kApplyTX, 8) helmholtz_apply_kernel(const z64* __restrict__ x, z64* __restrict__ y,
                                                                       const z64* __restrict__ b,
                                                                       const double* __restrict__ vel, StencilParams sp,
-                                                                      int k, int zFirst, int zSlab) {
-    const int x0 = blockIdx.x * kApplyTX, yy = blockIdx.y, zz = zFirst + (int)blockIdx.z;
+                                                                      int k, int px, int zFirst, int zSlab) {
+    const int x0 = blockIdx.x * px, yy = blockIdx.y, zz = zFirst + (int)blockIdx.z;
     const int64_t base = x0 + yy * (int64_t)sp.nx + (zz - zSlab) * ((int64_t)sp.nx * sp.ny);
-    ApplyRow(x, vel, sp, k, x0, yy, zz, base, [] {}, [&](int e, z64 v) {
+    ApplyRow(x, vel, sp, k, px, x0, yy, zz, base, [] {}, [&](int e, z64 v) {
         const int64_t idx = base * k + e;
         y[idx] = b ? b[idx] - v : v;
     });
@@ -120,9 +120,9 @@ __global__ void __launch_bounds__(kApplyTX, 8) helmholtz_apply_kernel(const z64*
 // the next has overwritten.  Bound by memory: 4 x 16 bytes per entry.
 __global__ void __launch_bounds__(kApplyTX, 8) helmholtz_in_place_kernel(z64* __restrict__ B, z64* __restrict__ ring,
                                                                          const double* __restrict__ vel,
-                                                                         StencilParams sp, int k, int zApply,
+                                                                         StencilParams sp, int k, int px, int zApply,
                                                                          int numApply, int zCopy, int ringPlanes) {
-    const int x0 = blockIdx.x * kApplyTX, yy = blockIdx.y;
+    const int x0 = blockIdx.x * px, yy = blockIdx.y;
     const bool apply = (int)blockIdx.z < numApply;
     const int zz = apply ? zApply + (int)blockIdx.z : zCopy + (int)blockIdx.z - numApply;
     const int64_t nxy = (int64_t)sp.nx * sp.ny, row = x0 + yy * (int64_t)sp.nx, base = row + zz * nxy;
@@ -132,10 +132,10 @@ __global__ void __launch_bounds__(kApplyTX, 8) helmholtz_in_place_kernel(z64* __
         PdlTrigger();
     };
     if (apply) {
-        ApplyRow(B, vel, sp, k, x0, yy, zz, base, ready, [&](int e, z64 v) { slot[e] = v; });
+        ApplyRow(B, vel, sp, k, px, x0, yy, zz, base, ready, [&](int e, z64 v) { slot[e] = v; });
     } else {
         ready();
-        const int n = min(kApplyTX, sp.nx - x0) * k;
+        const int n = min(px, sp.nx - x0) * k;
         for (int e = threadIdx.x; e < n; e += 4 * kApplyTX) {
             z64 v[4];
 #pragma unroll
@@ -602,6 +602,24 @@ unsigned ElementwiseGrid(int64_t n) { return (unsigned)std::min<int64_t>(CeilDiv
 
 // ---------------------------------------------------------------- host launchers
 
+// Points of a row per block: kApplyTX and a rest, or, where a launch would end on a
+// few long blocks, equal pieces: of at most kApplyTX points when it has less than
+// four waves of blocks (a wave is 8 per SM), of at most 32 when these have 3000
+// entries and more (from 24 columns on) or are less than half a wave.
+// 128 points and a rest -> equal pieces of up to 128 -> of up to 32 (us; 64 points on
+// 256 threads before): 129 x 40 x 40, k = 16: 50 -> 45 -> 49 (51), k = 64: 143 -> 120 ->
+// 115 (120); two planes of 127 x 40, k = 64: 36 -> 36 -> 22 (23), k = 16: 21 -> 21 -> 17
+// (19); 250 x 30 x 30, k = 48: 106 -> 106 -> 99 (100).  With more waves long pieces are
+// the better ones, and the short rest fills the gaps: 140 x 140 x 80, k = 8: 133 -> 136 ->
+// 167 (177), 220 x 220 x 40, k = 16: 252 -> 265 -> 306 (298).
+int ApplyPoints(int nx, int ny, int planes, int k) {
+    constexpr int64_t kWave = 8 * 148;
+    const int64_t blocks = (int64_t)CeilDiv(nx, kApplyTX) * ny * planes;
+    if (blocks >= 4 * kWave) return kApplyTX;
+    const int most = k >= 24 || blocks < kWave / 2 ? 32 : kApplyTX;
+    return (int)CeilDiv(nx, CeilDiv(nx, most));
+}
+
 void LaunchHelmholtzApply(const z64* x, z64* y, const z64* b, const double* vel, const StencilParams& sp, int k,
                           cudaStream_t st) {
     LaunchHelmholtzApplyPlanes(x, y, b, vel, sp, k, 0, sp.nz, 0, st);
@@ -609,8 +627,9 @@ void LaunchHelmholtzApply(const z64* x, z64* y, const z64* b, const double* vel,
 
 void LaunchHelmholtzApplyPlanes(const z64* x, z64* y, const z64* b, const double* vel, const StencilParams& sp,
                                 int k, int zFirst, int zCount, int zSlab, cudaStream_t st) {
-    dim3 grid(CeilDiv(sp.nx, kApplyTX), sp.ny, zCount);
-    helmholtz_apply_kernel<<<grid, kApplyTX, 0, st>>>(x, y, b, vel, sp, k, zFirst, zSlab);
+    const int px = ApplyPoints(sp.nx, sp.ny, zCount, k);
+    dim3 grid(CeilDiv(sp.nx, px), sp.ny, zCount);
+    helmholtz_apply_kernel<<<grid, kApplyTX, 0, st>>>(x, y, b, vel, sp, k, px, zFirst, zSlab);
     CUDA_LAUNCH_CHECK();
 }
 
@@ -633,12 +652,13 @@ void LaunchHelmholtzInPlace(z64* B, void* ring, const double* vel, const Stencil
     const int planes = InPlaceSlabPlanes(sp, k), slabs = (int)CeilDiv(sp.nz, planes);
     const int ringPlanes = std::min(sp.nz, 3 * planes);
     const int behind = slabs > 1 ? 2 : 1;
+    const int px = ApplyPoints(sp.nx, sp.ny, planes, k);
     auto count = [&](int s) { return s < 0 || s >= slabs ? 0 : std::min(planes, sp.nz - s * planes); };
     for (int s = 0; s < slabs + behind; ++s) {
         const int na = count(s), nc = count(s - behind);
         if (na + nc == 0) continue;
-        LaunchPdl(helmholtz_in_place_kernel, dim3(CeilDiv(sp.nx, kApplyTX), sp.ny, na + nc), dim3(kApplyTX), 0, st, B,
-                  static_cast<z64*>(ring), vel, sp, k, s * planes, na, (s - behind) * planes, ringPlanes);
+        LaunchPdl(helmholtz_in_place_kernel, dim3(CeilDiv(sp.nx, px), sp.ny, na + nc), dim3(kApplyTX), 0, st, B,
+                  static_cast<z64*>(ring), vel, sp, k, px, s * planes, na, (s - behind) * planes, ringPlanes);
         CUDA_LAUNCH_CHECK();
     }
 }
