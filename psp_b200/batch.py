@@ -15,8 +15,9 @@ every rank of an initialized ``torch.distributed`` process group (NCCL on
 GPUs, gloo on CPU), and the solutions are exchanged with all_gather_object.
 With ``streams > 1`` a rank keeps that many problems in flight at once, each
 on its own handle and CUDA stream (host threads; the library's calls release
-the interpreter lock), so the launches of small problems, which leave most
-SMs idle, overlap on the GPU.
+the interpreter lock), so that one problem's host work, set-up launches and
+panel solves of few tiles run beside another's.  A panel solve of more tiles than
+the GPU has SMs keeps all of them to its end.
 """
 import math
 from concurrent.futures import ThreadPoolExecutor

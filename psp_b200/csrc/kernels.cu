@@ -1,6 +1,6 @@
 // CUDA-core kernels of the solve: on-the-fly 7-point PML stencil, batched
-// complex GEMM over task lists, frontal LDL^T building blocks, multifrontal
-// gathers/scatters of the panel solves and the multi-RHS GMRES vector ops.
+// complex GEMM over task lists, frontal LDL^T building blocks and the multi-RHS
+// GMRES vector ops.  (The panel solves are in sweep_flow.cu and sweep_flow_tc.cu.)
 #include <algorithm>
 
 #include "kernels.cuh"

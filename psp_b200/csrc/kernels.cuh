@@ -1,7 +1,8 @@
 // Device kernels of the sweeping-preconditioned Helmholtz solve and the
-// descriptors the host orchestration fills for them.  Every batched kernel
-// walks a task list, so one launch covers all fronts of one elimination-tree
-// depth across every panel (and every problem) in flight.
+// descriptors the host orchestration fills for them.  Every batched
+// factorization kernel walks a task list, so one launch covers all fronts of one
+// elimination-tree depth across every panel in flight; a panel solve's list
+// covers the whole tree.
 #pragma once
 #include <vector>
 

@@ -131,8 +131,7 @@ __device__ void ProducerRole(const FlowFront<R>* __restrict__ fr, const FlowTile
     const int lane = threadIdx.x & 31;
     uint64_t policy;
     asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
-    TileSource<R> src;
-    src.Start(fr, tiles, n, w.ctrl, false);
+    TileSource<R> src(fr, tiles, n, w.ctrl);
     int g = 0;
     bool ok = true;
     for (int q = 0;; ++q) {

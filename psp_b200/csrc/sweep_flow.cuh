@@ -135,55 +135,31 @@ __device__ __forceinline__ void TmaLoadStream(void* dst, const void* tmap, int x
         : "memory");
 }
 
-// This CTA's tiles, by an atomic ticket (one warp).  A ticket and the words of
-// its tile and front are fetched a tile ahead, so that no load stalls the
-// copies: Next() returns the words of the next tile, one 16-byte word per
-// lane (front < 0: the list is done).
+// This CTA's tiles, by an atomic ticket (one warp).  Take() fetches the words of the
+// next tile and of its front, one 16-byte word per lane (front < 0: the list is done).
+// It takes the ticket when the copies of the tile before have been issued, and no
+// earlier: a CTA that runs ahead of its tiles by no more than its ring of stages
+// should hold no ticket that another CTA could start sooner.
 template <typename R>
 struct TileSource {
     const int4* tiles;
     const int4* fronts;
     int* ctrl;
-    int n, tk, tk1, next;
-    int4 ctx, ctx1;
+    int n, tk;
+    int4 ctx;
 
-    __device__ __forceinline__ int Ticket() { return (threadIdx.x & 31) == 0 ? atomicAdd(ctrl, 1) : 0; }
-    __device__ __forceinline__ int4 TileWords(int t) {
-        const int lane = threadIdx.x & 31;
-        return lane < kTileWords && t < n ? __ldg(tiles + (int64_t)t * kTileWords + lane) : make_int4(-1, 0, 0, 0);
-    }
-    // the front's words after those of the tile
-    __device__ __forceinline__ int4 FrontWords(int4 v, int t) {
-        const int lane = threadIdx.x & 31, front = __shfl_sync(~0u, v.x, 0);
-        if (lane >= kTileWords && lane < kCtxWords && t < n)
-            v = __ldg(fronts + (int64_t)front * kFrontWords + lane - kTileWords);
-        return v;
-    }
-    __device__ __forceinline__ void Start(const FlowFront<R>* fr, const FlowTile* tl, int n_, int* ctrl_, bool ahead) {
-        tiles = reinterpret_cast<const int4*>(tl);
-        fronts = reinterpret_cast<const int4*>(fr);
-        ctrl = ctrl_;
-        n = n_;
+    __device__ __forceinline__ TileSource(const FlowFront<R>* fr, const FlowTile* tl, int n_, int* ctrl_)
+        : tiles(reinterpret_cast<const int4*>(tl)), fronts(reinterpret_cast<const int4*>(fr)), ctrl(ctrl_), n(n_) {
         Take();
-        if (ahead) next = Ticket();  // lane 0's, read a tile later
     }
     __device__ __forceinline__ bool Done() const { return tk >= n; }
-    // Starts fetching the tile after the current one / makes it the current one.
-    __device__ __forceinline__ void Prefetch() {
-        tk1 = __shfl_sync(~0u, next, 0);
-        ctx1 = TileWords(tk1);
-        if (tk1 < n) next = Ticket();
-    }
-    // Takes the next tile now.  A CTA that runs ahead of its tiles by no more
-    // than its ring of stages should hold no ticket that another CTA could
-    // start sooner.
     __device__ __forceinline__ void Take() {
-        tk = __shfl_sync(~0u, Ticket(), 0);
-        ctx = FrontWords(TileWords(tk), tk);
-    }
-    __device__ __forceinline__ void Advance() {
-        tk = tk1;
-        ctx = FrontWords(ctx1, tk);
+        const int lane = threadIdx.x & 31;
+        tk = __shfl_sync(~0u, lane == 0 ? atomicAdd(ctrl, 1) : 0, 0);
+        ctx = lane < kTileWords && tk < n ? __ldg(tiles + (int64_t)tk * kTileWords + lane) : make_int4(-1, 0, 0, 0);
+        const int front = __shfl_sync(~0u, ctx.x, 0);
+        if (lane >= kTileWords && lane < kCtxWords && tk < n)
+            ctx = __ldg(fronts + (int64_t)front * kFrontWords + lane - kTileWords);
     }
 };
 

@@ -117,8 +117,7 @@ __device__ void ProducerRole(const FlowFront<float>* __restrict__ fr, const Flow
     const int lane = threadIdx.x & 31;
     uint64_t policy;
     asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
-    TileSource<float> src;
-    src.Start(fr, tiles, n, w.ctrl, false);
+    TileSource<float> src(fr, tiles, n, w.ctrl);
     int g = 0;
     for (int q = 0;; ++q) {
         const int qs = q % kQueue;
