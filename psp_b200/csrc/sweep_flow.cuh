@@ -16,15 +16,14 @@ constexpr int kTileWords = sizeof(FlowTile) / 16, kFrontWords = sizeof(FlowFront
 constexpr int kCtxWords = kTileWords + kFrontWords;
 static_assert(sizeof(FlowFront<float>) == sizeof(FlowFront<double>) && kCtxWords <= 32, "copied in 16-byte words");
 
-
-// Bounded wait on one phase of an mbarrier; false once this or another role of
-// the CTA (S.abort) gave up.
-template <typename Sync>
-__device__ __forceinline__ bool Wait(uint64_t* mbar, uint32_t parity, Sync& S, int* status) {
-    if (umma::MbarTryWait(mbar, parity)) return true;
+// Repeats a test until it holds, the CTA gave up, or the wait has run out (which
+// gives up).
+template <typename Sync, typename Test>
+__device__ __forceinline__ bool WaitUntil(const Test& test, Sync& S, int* status) {
+    if (test()) return true;
     const uint64_t t0 = umma::GlobalTimerNs();
     for (;;) {
-        if (umma::MbarTryWait(mbar, parity)) return true;
+        if (test()) return true;
         if (*reinterpret_cast<volatile int*>(&S.abort)) return false;
         if (umma::GlobalTimerNs() - t0 > umma::kWaitLimitNs) break;
     }
@@ -33,10 +32,23 @@ __device__ __forceinline__ bool Wait(uint64_t* mbar, uint32_t parity, Sync& S, i
     return false;
 }
 
+// Bounded wait on one phase of an mbarrier; false once this or another role of
+// the CTA (S.abort) gave up.
+template <typename Sync>
+__device__ __forceinline__ bool Wait(uint64_t* mbar, uint32_t parity, Sync& S, int* status) {
+    return WaitUntil([&] { return umma::MbarTryWait(mbar, parity); }, S, status);
+}
+
 // The same by a whole warp, which goes on or gives up together.
 template <typename Sync>
 __device__ __forceinline__ bool WaitWarp(uint64_t* mbar, uint32_t parity, Sync& S, int* status) {
     return __all_sync(~0u, Wait(mbar, parity, S, status));
+}
+
+__device__ __forceinline__ int LoadAcquire(const int* p) {
+    int v;
+    asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
 }
 
 // Whether both counters of a pair have reached what a tile needs.
@@ -53,21 +65,8 @@ __device__ __forceinline__ bool CountsReached(const int* pair, int need0, int ne
 template <typename Sync>
 __device__ __forceinline__ bool TileReady(const FlowTile& t, bool wait, Sync& S, const FlowWork& w) {
     if (t.dep < 0) return true;
-    const int* const pair = w.done + t.dep;
-    bool ok = CountsReached(pair, t.need0, t.need1);
-    if (wait && !ok) {
-        const uint64_t t0 = umma::GlobalTimerNs();
-        for (;;) {
-            ok = CountsReached(pair, t.need0, t.need1);
-            if (ok || *reinterpret_cast<volatile int*>(&S.abort)) break;
-            if (umma::GlobalTimerNs() - t0 > umma::kWaitLimitNs) {
-                *reinterpret_cast<volatile int*>(&S.abort) = 1;
-                atomicOr(w.status, 2);
-                break;
-            }
-        }
-    }
-    return __all_sync(~0u, ok);
+    auto reached = [&] { return CountsReached(w.done + t.dep, t.need0, t.need1); };
+    return __all_sync(~0u, wait ? WaitUntil(reached, S, w.status) : reached());
 }
 
 // Global data written by other CTAs of this launch: through L2.
