@@ -38,8 +38,8 @@
 // updates and the grid written on the way out a tile's write-out took 5 us
 // instead of 3, and with tickets taken two tiles ahead the narrow levels were
 // badly balanced (39 instead of 29 ms then per sweep at 116^3).  Measured against one
-// launch per level and direction, whole sweeps: 116^3, k = 16: 44.1 -> 27.2 ms
-// (1.9 TB/s of factors); 96 x 96 x 76, k = 32: 34.7 -> 16.9 ms.
+// launch per level and direction, whole sweeps: 116^3, k = 16: 44.1 -> 26.9 ms
+// (1.9 TB/s of factors); 96 x 96 x 76, k = 32: 34.7 -> 16.7 ms.
 #include <algorithm>
 
 #include "sweep_flow.cuh"
